@@ -273,11 +273,11 @@ bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t* vals_in, 
 
 /* Walk autotuner (no counterpart in the reference, whose walk is one serial loop). Times each
  * launch shape of the quadrupole tree walk (warps per block, register budget as resident blocks
- * per SM, per-warp stack depth, cell-evaluation form, and bodies per warp group: 32, or 16 / 8
- * for a single system, where more and smaller groups fill the GPU at small N; a group never
- * exceeds the 32 lanes of a warp, whose opening masks are 32-bit; ensembles walk their fixed
- * table of groups of up to 32) on the tree currently in the context: the last bh_step /
- * bh_build, or the last bh_batch_step of an ensemble. Each shape runs `trials` timed
+ * per SM, per-warp stack depth, cell-evaluation form, and bodies per warp group: shape 0, the
+ * default, takes 32, 16, 8 or 4 by the number of bodies, shapes 8 to 11 fix 16 or 8, the others 32;
+ * a group never exceeds the 32 lanes of a warp, whose opening masks are 32-bit; ensembles walk
+ * their fixed table of groups, sized by their number of bodies in all) on the tree currently in
+ * the context: the last bh_step / bh_build, or the last bh_batch_step of an ensemble. Each shape runs `trials` timed
  * force-only walks after one warm-up (the state is not changed); the fastest median becomes the
  * context's walk for quadrupole steps with eps > 0. Shapes whose stack cannot hold the tree get
  * ms = -1. */

@@ -1064,14 +1064,17 @@ bh_status batch_layout(bh_ctx* c, const uint32_t* sys_offsets, size_t nsys) {
   if (!c->body_sys) BH_TRY(dalloc(&c->body_sys, c->cap));
   std::vector<uint16_t> bs(n);
   std::vector<int4> groups;
+  const uint32_t gsize = (uint32_t)walk_group_size(n);
   for (size_t s = 0; s < nsys; ++s) {
     const uint32_t b0 = sys_offsets[s], b1 = sys_offsets[s + 1];
     for (uint32_t i = b0; i < b1; ++i) bs[i] = (uint16_t)s;
-    for (uint32_t g = b0; g < b1; g += 32) groups.push_back(make_int4((int)g, (int)std::min(32u, b1 - g), (int)s, (int)s));
+    for (uint32_t g = b0; g < b1; g += gsize)
+      groups.push_back(make_int4((int)g, (int)std::min(gsize, b1 - g), (int)s, (int)s));
   }
   dfree(c->groups);
   BH_TRY(dalloc(&c->groups, groups.size()));
   c->ngroups = (int)groups.size();
+  c->batch_group = (int)gsize;
   cudaMemcpyAsync(c->sys_off, sys_offsets, sizeof(uint32_t) * (nsys + 1), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->body_sys, bs.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->groups, groups.data(), sizeof(int4) * groups.size(), cudaMemcpyHostToDevice, c->stream);
@@ -1257,13 +1260,13 @@ bh_status bh_autotune_walk(bh_ctx* c, double theta, double eps, int trials, bh_t
   float best_ms = 0.f;
   int best = 0;
   for (int v = 0; v < nv; ++v) {
-    const bh::WalkVariant info = bh::walk_variant_info(v);
+    const bh::WalkVariant info = bh::walk_variant_info(v, c->n);
     out->warps_per_block[v] = info.warps;
     out->min_blocks_per_sm[v] = info.min_blocks;
     out->stack_depth[v] = info.stack;
     out->cell_form[v] = info.form;
     out->registers[v] = info.regs;
-    out->group_size[v] = batch ? 32 : info.group;  // ensembles walk their fixed group table
+    out->group_size[v] = batch ? c->batch_group : info.group;  // ensembles walk their fixed group table
     std::vector<float> ms;
     uint32_t e = 0;
     for (int t = 0; t <= trials && e == 0; ++t) {  // trial 0 warms up

@@ -181,6 +181,7 @@ struct bh_ctx {
   bh::Geom* sys_geom = nullptr;    // device [nsys]
   int4* groups = nullptr;          // device walk groups: first body, body count, root node, system
   int ngroups = 0;
+  int batch_group = 32;            // largest group of the table (32, 16, 8 or 4)
   size_t sys_cap = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // captured batched step, by state parity
   bh_params graph_params = {};
@@ -285,7 +286,9 @@ struct WalkVariant {
   int warps, min_blocks, stack, form, regs, group;  // group: bodies per warp (single systems)
 };
 int walk_variants();
-WalkVariant walk_variant_info(int v);
+WalkVariant walk_variant_info(int v, size_t n);
+// Bodies per walk group for n bodies in all (a single system, or the systems of an ensemble).
+int walk_group_size(size_t n);
 void launch_walk_variant(bh_ctx* c, int v, int n, float theta, float eps, float4* acc_out, bool batch);
 
 // Frees the differentiable-path state of the context.

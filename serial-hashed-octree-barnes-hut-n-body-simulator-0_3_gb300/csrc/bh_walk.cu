@@ -1,7 +1,9 @@
 // Tree walk + force: ComputeHOTOctreeForce / TraverseHOTInteractionList /
 // ComputeHOTForceInteractionList / LinearHashedOctree::MAC (src/HashedOctree.hpp:262-459,
 // src/HashedOctree.cpp:872-885), one warp per group of up to 32 consecutive bodies in tree order
-// (32 by default; the autotuner may pick 16 or 8 for small single systems).
+// (32, 16, 8 or 4 by the number of bodies: walk_group_size). A group of G < 32 bodies fills the warp
+// 32 / G times: lane l holds body l % G, and the 32 / G slots of G lanes take different entries of
+// the evaluation and different children of the per-lane opening test, so no lane idles.
 //
 // Per-lane exactness. The reference walks each body separately: pop a node; test each
 // existing child with the MAC size^2 / d^2 < theta^2 against the body; accepted children go
@@ -116,13 +118,15 @@ __device__ __forceinline__ void record_chunk(const Rec& r, int kind, int cnt, co
 }
 
 // 32 multipole cells (monopole + quadrupole). The lane mask rides in st2.w.
-template <bool kRec, int kForm = 0, class Smem>
-__device__ __forceinline__ void eval_cells(Smem& s, int cnt, const WalkNode* __restrict__ nodes,
-                                           uint32_t lanebit, float px, float py, float pz, float eps2, Acc& acc,
+template <bool kRec, int kForm, int kGroup, class Smem>
+__device__ __forceinline__ void eval_cells(Smem& s, int cnt, const WalkNode* __restrict__ nodes, int lane,
+                                           float px, float py, float pz, float eps2, Acc& acc,
                                            unsigned long long& ev, const Rec& rec) {
-  ev += (unsigned)cnt;
+  constexpr int kSlots = 32 / kGroup;
+  const int slot = lane / kGroup;
+  const uint32_t lanebit = 1u << (lane % kGroup);
+  ev += (unsigned)(cnt + kSlots - 1) / kSlots;
   __syncwarp();
-  const int lane = __ffs(lanebit) - 1;
   if (kRec) record_chunk(rec, 0, cnt, s.cell_node, s.cell_mask, lane);
   if (lane < cnt) {
     const WalkNode* nd = nodes + s.cell_node[lane];
@@ -131,14 +135,17 @@ __device__ __forceinline__ void eval_cells(Smem& s, int cnt, const WalkNode* __r
     float4 q2 = __ldg(&nd->q2);
     q2.w = __uint_as_float(s.cell_mask[lane]);
     s.st2[lane] = q2;
+  } else if (kSlots > 1) {  // a slot may run past the last entry: empty mask, finite terms
+    s.st0[lane] = s.st1[lane] = s.st2[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncwarp();
   float bx = 0.f, by = 0.f, bz = 0.f;
   // unroll factors measured at N = 2^22: cells 2 / 4 / 8 / 12 / 16 / 32 -> walk 17.98 / 17.45 /
   // 17.71 / 17.44 / 17.37 / 17.44 ms; points 2 / 4 / 8 / 16 (cells at 16) -> 17.46 / 17.37 /
   // 17.31 / 17.67 ms
-#pragma unroll 16
-  for (int j = 0; j < cnt; ++j) {
+#pragma unroll(16 / kSlots > 2 ? 16 / kSlots : 2)
+  for (int r = 0; r < cnt; r += kSlots) {
+    const int j = r + slot;
     const float4 c0 = s.st0[j], c1 = s.st1[j], c2 = s.st2[j];
     const float dx = c0.x - px, dy = c0.y - py, dz = c0.z - pz;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
@@ -175,13 +182,15 @@ __device__ __forceinline__ void eval_cells(Smem& s, int cnt, const WalkNode* __r
 }
 
 // Up to 32 point masses. The lane mask is read from pt_mask.
-template <bool kSelfTest, bool kRec, class Smem>
+template <bool kSelfTest, bool kRec, int kGroup, class Smem>
 __device__ __forceinline__ void eval_points(Smem& s, int cnt, const WalkNode* __restrict__ nodes,
-                                            const float4* __restrict__ tpos, uint32_t lanebit, float px, float py,
+                                            const float4* __restrict__ tpos, int lane, float px, float py,
                                             float pz, float eps2, Acc& acc, unsigned long long& ev, const Rec& rec) {
-  ev += (unsigned)cnt;
+  constexpr int kSlots = 32 / kGroup;
+  const int slot = lane / kGroup;
+  const uint32_t lanebit = 1u << (lane % kGroup);
+  ev += (unsigned)(cnt + kSlots - 1) / kSlots;
   __syncwarp();
-  const int lane = __ffs(lanebit) - 1;
   if (kRec) record_chunk(rec, 1, cnt, s.pt_idx, s.pt_mask, lane);
   if (lane < cnt) {
     const int e = s.pt_idx[lane];
@@ -194,11 +203,15 @@ __device__ __forceinline__ void eval_points(Smem& s, int cnt, const WalkNode* __
       v = make_float4(mac.x, mac.y, mac.z, __ldg(&nd->mq.x));
     }
     s.st0[lane] = v;
+  } else if (kSlots > 1) {  // a slot may run past the last entry
+    s.st0[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+    s.pt_mask[lane] = 0u;
   }
   __syncwarp();
   float bx = 0.f, by = 0.f, bz = 0.f;
-#pragma unroll 8
-  for (int j = 0; j < cnt; ++j) {
+#pragma unroll(8 / kSlots > 2 ? 8 / kSlots : 2)
+  for (int r = 0; r < cnt; r += kSlots) {
+    const int j = r + slot;
     const float4 v = s.st0[j];
     const uint32_t mk = s.pt_mask[j];
     const float dx = v.x - px, dy = v.y - py, dz = v.z - pz;
@@ -234,14 +247,14 @@ __device__ __forceinline__ void shift_down(int* idx, uint32_t* msk, int n, int l
   }
 }
 
-template <bool kQuad, bool kSelfTest, bool kRec = false, class Cfg = CfgDefault>
+template <bool kQuad, bool kSelfTest, bool kRec = false, class Cfg = CfgDefault, int kGroup = 32>
 __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const WalkNode* __restrict__ nodes,
                                                    const float4* __restrict__ tpos,
                                                    const uint32_t* __restrict__ tslot, int n, float theta2,
                                                    float eps2, float4* __restrict__ acc_slot,
                                                    float4* __restrict__ vel_kick, float half_dt,
                                                    float4* __restrict__ vel_copy,
-                                                   const int4* __restrict__ groups, int ngroups_table, int gsize,
+                                                   const int4* __restrict__ groups, int ngroups_table,
                                                    Counters* __restrict__ ctr, uint32_t* __restrict__ err,
                                                    Chunk* __restrict__ tape = nullptr,
                                                    unsigned* __restrict__ tape_count = nullptr, int tape_cap = 0) {
@@ -252,20 +265,32 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
   const uint32_t lt_mask = lanebit - 1u;
   WarpSmemT<kStack>& s = smem[threadIdx.x >> 5];
   if (*((volatile uint32_t*)err) & (kErrNodes | kErrTimeout)) return;
-  // work items: groups of up to 32 consecutive bodies (tree order) under one root. Without a
-  // group table, group g is bodies [gsize g, gsize g + gsize) of the single tree rooted at node 0
-  // (gsize <= 32; lanes beyond the group's bodies stay out of every mask); batched ensembles pass
-  // (first body, body count, root node) per group.
-  const int ngroups = groups ? ngroups_table : (n + gsize - 1) / gsize;
+  // work items: groups of up to kGroup consecutive bodies (tree order) under one root. Without a
+  // group table, group g is bodies [kGroup g, kGroup g + kGroup) of the single tree rooted at node
+  // 0; batched ensembles pass (first body, body count, root node) per group. Lane l holds body
+  // l % kGroup of its group; the 32 / kGroup slots of lanes with the same bodies take different
+  // entries in the evaluation and different children in the per-lane MAC.
+  constexpr int kSlots = 32 / kGroup;
+  const int slot = lane / kGroup, glane = lane % kGroup;
+  const int ngroups = groups ? ngroups_table : (n + kGroup - 1) / kGroup;
   const float acc_scale = theta2 * (1.f - kMacMargin);
   const float open_scale = theta2 * (1.f + kMacMargin);
   unsigned long long tot_cell = 0, tot_pt = 0, ev_cell = 0, ev_pt = 0;  // ev_*: warp-uniform
   bool overflow = false;
 
+  // Groups come from a queue. With small groups (few of them: see walk_group_size) a warp's first
+  // one goes by its place in the grid, warp 0 of every block first, so that they spread over all the
+  // SMs (16 384 bodies in groups of 8: 210 -> 171 us); with groups of 32 neighbouring groups share a
+  // block's L1, and the queue alone is faster (2^22 bodies: 17.2 against 18.1 ms).
+  bool queued = kGroup == 32;
   for (;;) {
-    int g = 0;
-    if (lane == 0) g = (int)atomicAdd(&ctr->group_next, 1u);
-    g = __shfl_sync(0xffffffffu, g, 0);
+    int g = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
+    if (queued) {
+      if (lane == 0) g = (int)atomicAdd(&ctr->group_next, 1u);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (kGroup < 32) g += (int)gridDim.x * Cfg::kWarps;
+    }
+    queued = true;
     if (g >= ngroups) break;
     int gbase, gcount, root;
     if (groups) {
@@ -274,20 +299,20 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
       gcount = gr.y;
       root = gr.z;
     } else {
-      gbase = g * gsize;
-      gcount = min(gsize, n - gbase);
+      gbase = g * kGroup;
+      gcount = min(kGroup, n - gbase);
       root = 0;
     }
     const int4 root_link = __ldg(&nodes[root].link);
     const Rec rec{tape, tape_count, tape_cap, gbase, gcount, err};
-    const int i = gbase + lane;
-    const bool valid = lane < gcount;
+    const int i = gbase + glane;
+    const bool valid = glane < gcount;
     const float4 p = __ldg(tpos + (valid ? i : gbase));
-    const uint32_t active = __ballot_sync(0xffffffffu, valid);
+    const uint32_t active = gcount >= 32 ? 0xffffffffu : (1u << gcount) - 1u;
     // bounding box of the group's bodies
     float bminx = p.x, bminy = p.y, bminz = p.z, bmaxx = p.x, bmaxy = p.y, bmaxz = p.z;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = kGroup / 2; o > 0; o >>= 1) {
       bminx = fminf(bminx, __shfl_xor_sync(0xffffffffu, bminx, o));
       bminy = fminf(bminy, __shfl_xor_sync(0xffffffffu, bminy, o));
       bminz = fminf(bminz, __shfl_xor_sync(0xffffffffu, bminz, o));
@@ -311,7 +336,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           s.pt_mask[lane] = active;
         }
         if (lane == 0) cnt_pt += (long long)k * __popc(active);
-        eval_points<kSelfTest, kRec>(s,k, nodes, tpos, lanebit, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+        eval_points<kSelfTest, kRec, kGroup>(s, k, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
       }
       if (lane == 0) cnt_pt -= __popc(active);
     } else {
@@ -384,7 +409,24 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
       // and sizes are staged in shared memory (one broadcast load per child), and the child's
       // own lane applies its open mask to the ballot
       uint32_t mixed_bits = __ballot_sync(0xffffffffu, mixed);
-      if (mixed_bits) {
+      if (kSlots > 1 && mixed_bits) {
+        // one mixed child per slot and round: the children packed to the front of the staging row
+        const int nm = __popc(mixed_bits), my = __popc(mixed_bits & lt_mask);
+        __syncwarp();
+        if (mixed) s.st0[my] = make_float4(mac.x, mac.y, mac.z, fabsf(mac.w));
+        __syncwarp();
+        for (int r = 0; r < nm; r += kSlots) {
+          const float4 cm = s.st0[min(r + slot, nm - 1)];
+          const float dx = cm.x - p.x, dy = cm.y - p.y, dz = cm.z - p.z;
+          const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          const uint32_t a = __ballot_sync(0xffffffffu, cm.w < theta2 * d2);
+          if (mixed && my >= r && my < r + kSlots) {
+            const uint32_t mine = a >> ((my - r) * kGroup);  // pmask holds kGroup bits
+            am = mine & pmask;
+            om = pmask & ~mine;
+          }
+        }
+      } else if (mixed_bits) {
         __syncwarp();
         if (mixed) s.st0[lane] = make_float4(mac.x, mac.y, mac.z, fabsf(mac.w));
         __syncwarp();
@@ -421,7 +463,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           }
           ncell += __popc(bal);
           if (ncell >= 32) {
-            eval_cells<kRec, Cfg::kForm>(s,32, nodes, lanebit, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
+            eval_cells<kRec, Cfg::kForm, kGroup>(s, 32, nodes, lane, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
             shift_down(s.cell_node, s.cell_mask, ncell, lane);
             ncell -= 32;
           }
@@ -439,7 +481,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           }
           npt += __popc(bal);
           if (npt >= 32) {
-            eval_points<kSelfTest, kRec>(s,32, nodes, tpos, lanebit, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+            eval_points<kSelfTest, kRec, kGroup>(s, 32, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
             shift_down(s.pt_idx, s.pt_mask, npt, lane);
             npt -= 32;
           }
@@ -504,7 +546,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
             }
             npt += kk;
             if (npt >= 32) {
-              eval_points<kSelfTest, kRec>(s,32, nodes, tpos, lanebit, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+              eval_points<kSelfTest, kRec, kGroup>(s, 32, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
               shift_down(s.pt_idx, s.pt_mask, npt, lane);
               npt -= 32;
             }
@@ -513,21 +555,34 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         }
       }
     }
-    if (ncell > 0) eval_cells<kRec, Cfg::kForm>(s,ncell, nodes, lanebit, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
-    if (npt > 0) eval_points<kSelfTest, kRec>(s,npt, nodes, tpos, lanebit, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
-    if (valid) {
-      const uint32_t slot = __ldg(tslot + i);
+    if (ncell > 0) eval_cells<kRec, Cfg::kForm, kGroup>(s, ncell, nodes, lane, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
+    if (npt > 0) eval_points<kSelfTest, kRec, kGroup>(s, npt, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+    if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
+#pragma unroll
+      for (int o = kGroup; o < 32; o <<= 1) {
+        const float ox = __shfl_xor_sync(0xffffffffu, acc.sx, o), oy = __shfl_xor_sync(0xffffffffu, acc.sy, o),
+                    oz = __shfl_xor_sync(0xffffffffu, acc.sz, o);
+        const float ex = __shfl_xor_sync(0xffffffffu, acc.cx, o), ey = __shfl_xor_sync(0xffffffffu, acc.cy, o),
+                    ez = __shfl_xor_sync(0xffffffffu, acc.cz, o);
+        acc.cx += ex;
+        acc.cy += ey;
+        acc.cz += ez;
+        acc.add(ox, oy, oz);
+      }
+    }
+    if (valid && slot == 0) {
+      const uint32_t bslot = __ldg(tslot + i);
       const float ax = acc.sx, ay = acc.sy, az = acc.sz;
-      acc_slot[slot] = make_float4(ax, ay, az, 0.f);
+      acc_slot[bslot] = make_float4(ax, ay, az, 0.f);
       if (vel_kick) {
-        float4 v = vel_kick[slot];
+        float4 v = vel_kick[bslot];
         v.x += ax * half_dt;
         v.y += ay * half_dt;
         v.z += az * half_dt;
-        vel_kick[slot] = v;
+        vel_kick[bslot] = v;
         // a second copy of the kicked velocity (the caller's mapped pinned buffer of a host-IO
         // step: the download then rides on the walk instead of following it)
-        if (vel_copy) vel_copy[slot] = v;
+        if (vel_copy) vel_copy[bslot] = v;
       }
     }
     tot_cell += (unsigned long long)cnt_cell;
@@ -555,7 +610,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
 // Persistent grid of one walk instantiation on the current device: every block that can be
 // resident at once (kept per device; bh_create fills it through walk_init before any capture).
 constexpr int kWalkMaxDevices = 64;
-template <bool kQuad, bool kSelf, bool kRec, class Cfg>
+template <bool kQuad, bool kSelf, bool kRec, class Cfg, int kGroup = 32>
 int walk_grid() {
   static int blocks[kWalkMaxDevices] = {};
   int dev = 0;
@@ -566,20 +621,38 @@ int walk_grid() {
   if (blocks[dev] == 0) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk<kQuad, kSelf, kRec, Cfg>, Cfg::kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk<kQuad, kSelf, kRec, Cfg, kGroup>, Cfg::kThreads, 0);
     blocks[dev] = max(1, sms * max(1, per_sm));
   }
   return blocks[dev];
 }
 
+struct WalkArgs {
+  float theta2, eps2, half_dt;
+  float4 *acc_slot, *vel_kick, *vel_copy;
+  bool batch;
+};
+
+template <bool kQuad, bool kSelf, class Cfg = CfgDefault, int kGroup = 32>
+void launch_walk_t(bh_ctx* c, int n, const WalkArgs& a) {
+  const int ngroups = a.batch ? c->ngroups : (n + kGroup - 1) / kGroup;
+  // every resident block, or a block per group when there are fewer groups than that: the warps
+  // that find no group leave, the others spread over all the SMs
+  const int grid = min(walk_grid<kQuad, kSelf, false, Cfg, kGroup>(), ngroups);
+  k_walk<kQuad, kSelf, false, Cfg, kGroup><<<grid, Cfg::kThreads, 0, c->stream>>>(
+      c->wnode, c->tpos, c->tslot, n, a.theta2, a.eps2, a.acc_slot, a.vel_kick, a.half_dt, a.vel_copy,
+      a.batch ? c->groups : nullptr, c->ngroups, c->counters, c->err);
+}
+
+// The walk with groups of `group` bodies (32, 16, 8 or 4; an ensemble's table is built for it).
 template <bool kQuad, bool kSelf, class Cfg = CfgDefault>
-void launch_walk_t(bh_ctx* c, int n, float theta2, float eps2, float4* acc_slot, float4* vel_kick, float half_dt,
-                   float4* vel_copy, bool batch, int gsize = 32) {
-  const int ngroups = batch ? c->ngroups : (n + gsize - 1) / gsize;
-  const int grid = min(walk_grid<kQuad, kSelf, false, Cfg>(), ngroups / Cfg::kWarps + 1);
-  k_walk<kQuad, kSelf, false, Cfg><<<grid, Cfg::kThreads, 0, c->stream>>>(
-      c->wnode, c->tpos, c->tslot, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch ? c->groups : nullptr,
-      c->ngroups, gsize, c->counters, c->err);
+void launch_walk_group(bh_ctx* c, int n, const WalkArgs& a, int group) {
+  switch (group) {
+    case 4: launch_walk_t<kQuad, kSelf, Cfg, 4>(c, n, a); break;
+    case 8: launch_walk_t<kQuad, kSelf, Cfg, 8>(c, n, a); break;
+    case 16: launch_walk_t<kQuad, kSelf, Cfg, 16>(c, n, a); break;
+    default: launch_walk_t<kQuad, kSelf, Cfg, 32>(c, n, a); break;
+  }
 }
 
 // Launch shapes the autotuner chooses from for the quadrupole walk with positive softening
@@ -592,45 +665,55 @@ using Cfg4 = WalkCfg<4, 6, 384>;
 using Cfg5 = WalkCfg<4, 8, 512>;
 using Cfg6 = WalkCfg<8, 4, 384, 1>;
 using Cfg7 = WalkCfg<4, 8, 384, 1>;
-// variants 8 and 9: the default shape with groups of 16 and 8 bodies (single systems; more,
-// smaller groups fill the GPU when N is small)
-// variants 10 and 11: 104 registers (two 8-warp blocks per SM) with groups of 16 and 8 bodies:
-// small single systems, where a few warps per SM walk and the walk's time is one warp's chain of
-// dependent latencies, which more registers let the compiler overlap
+// Variant 0, the default, takes its group size from the number of bodies (walk_group_size);
+// variants 8 and 9 fix it to 16 and 8, and 10 and 11 do so at 104 registers (two 8-warp blocks per
+// SM): small single systems, where a few warps per SM walk and the walk's time is one warp's chain
+// of dependent latencies. Ensembles walk their fixed table, whatever the variant's group.
 constexpr int kVariants = 12;
 
-template <class Cfg>
-WalkVariant variant_info(int group = 32) {
+// The 104-register shape of the small groups, while about one wave of its blocks (16 warps per SM)
+// holds them all: a warp then walks one group, and its latency is the walk's. Quadrupole walk, us at
+// 64 / 104 registers: 1 000 bodies in groups of 4 54.3 / 51.6; 10 000 (2 500 groups) 123.7 / 117.9;
+// 16 384 in groups of 8 171.5 / 160.7, of 4 (4 096 groups) 182.8 / 197.0; 65 536 in groups of 16
+// (4 096 groups) 402 / 406.
+constexpr int kWideMaxGroups = 3072;
+bool walk_wide(int ngroups, int group) { return group < 32 && ngroups <= kWideMaxGroups; }
+
+template <class Cfg, int kGroup = 32>
+WalkVariant variant_info() {
   cudaFuncAttributes fa{};
-  cudaFuncGetAttributes(&fa, k_walk<true, false, false, Cfg>);
-  return {Cfg::kWarps, Cfg::kMinBlocks, Cfg::kStack, Cfg::kForm, fa.numRegs, group};
+  cudaFuncGetAttributes(&fa, k_walk<true, false, false, Cfg, kGroup>);
+  return {Cfg::kWarps, Cfg::kMinBlocks, Cfg::kStack, Cfg::kForm, fa.numRegs, kGroup};
 }
 
-void launch_quad_variant(bh_ctx* c, int v, int n, float theta2, float eps2, float4* acc_slot, float4* vel_kick,
-                         float half_dt, float4* vel_copy, bool batch) {
+// The default shape at a group size: 104 registers while the groups are few (see walk_wide).
+void launch_quad_default(bh_ctx* c, int n, const WalkArgs& a, int group) {
+  if (walk_wide(a.batch ? c->ngroups : (n + group - 1) / group, group))
+    launch_walk_group<true, false, Cfg2>(c, n, a, group);
+  else
+    launch_walk_group<true, false>(c, n, a, group);
+}
+
+void launch_quad_variant(bh_ctx* c, int v, int n, const WalkArgs& a) {
+  const int table = a.batch ? c->batch_group : 0;
+  if (a.batch && table != 32) {  // small ensembles: the table's own group size, default shape
+    launch_quad_default(c, n, a, table);
+    return;
+  }
+  if (a.batch && v >= 8) v = 0;
   switch (v) {
-    case 1: launch_walk_t<true, false, Cfg1>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 2: launch_walk_t<true, false, Cfg2>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 3: launch_walk_t<true, false, Cfg3>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 4: launch_walk_t<true, false, Cfg4>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 5: launch_walk_t<true, false, Cfg5>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 6: launch_walk_t<true, false, Cfg6>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 7: launch_walk_t<true, false, Cfg7>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch); break;
-    case 8:
-      launch_walk_t<true, false, CfgDefault>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, 16);
-      break;
-    case 9:
-      launch_walk_t<true, false, CfgDefault>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, 8);
-      break;
-    case 10:
-      launch_walk_t<true, false, Cfg2>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, 16);
-      break;
-    case 11:
-      launch_walk_t<true, false, Cfg2>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, 8);
-      break;
-    default:
-      launch_walk_t<true, false, CfgDefault>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch);
-      break;
+    case 1: launch_walk_t<true, false, Cfg1>(c, n, a); break;
+    case 2: launch_walk_t<true, false, Cfg2>(c, n, a); break;
+    case 3: launch_walk_t<true, false, Cfg3>(c, n, a); break;
+    case 4: launch_walk_t<true, false, Cfg4>(c, n, a); break;
+    case 5: launch_walk_t<true, false, Cfg5>(c, n, a); break;
+    case 6: launch_walk_t<true, false, Cfg6>(c, n, a); break;
+    case 7: launch_walk_t<true, false, Cfg7>(c, n, a); break;
+    case 8: launch_walk_t<true, false, CfgDefault, 16>(c, n, a); break;
+    case 9: launch_walk_t<true, false, CfgDefault, 8>(c, n, a); break;
+    case 10: launch_walk_t<true, false, Cfg2, 16>(c, n, a); break;
+    case 11: launch_walk_t<true, false, Cfg2, 8>(c, n, a); break;
+    default: launch_quad_default(c, n, a, a.batch ? 32 : walk_group_size(n)); break;
   }
 }
 
@@ -638,7 +721,19 @@ void launch_quad_variant(bh_ctx* c, int v, int n, float theta2, float eps2, floa
 
 int walk_variants() { return kVariants; }
 
-WalkVariant walk_variant_info(int v) {
+// Small groups give more warps and, with their boxes, fewer entries a body (at 16 384 bodies, leaf
+// capacity 1, a group of 32 / 16 / 8 evaluates 2200 / 1835 / 1569 entries), but each group traverses
+// the tree. Quadrupole walk, us with groups of 4 / 8 / 16 / 32 (theta 0.5): 1 000 bodies 52 / 58 / 68 /
+// 134; 10 000 118 / 126 / 159 / 304; 16 384 183 / 161 / 179 / 345; 32 768 298 / 259 / 240 / 351;
+// 65 536 576 / 419 / 402 / 452; 131 072 1104 / 769 / 642 / 741; 262 144 2269 / 1507 / 1210 / 1206.
+// The literal walk crosses at the same sizes.
+int walk_group_size(size_t n) {
+  if (n < 12288) return 4;
+  if (n < 24576) return 8;
+  return n < 196608 ? 16 : 32;
+}
+
+WalkVariant walk_variant_info(int v, size_t n) {
   switch (v) {
     case 1: return variant_info<Cfg1>();
     case 2: return variant_info<Cfg2>();
@@ -647,11 +742,17 @@ WalkVariant walk_variant_info(int v) {
     case 5: return variant_info<Cfg5>();
     case 6: return variant_info<Cfg6>();
     case 7: return variant_info<Cfg7>();
-    case 8: return variant_info<CfgDefault>(16);
-    case 9: return variant_info<CfgDefault>(8);
-    case 10: return variant_info<Cfg2>(16);
-    case 11: return variant_info<Cfg2>(8);
-    default: return variant_info<CfgDefault>();
+    case 8: return variant_info<CfgDefault, 16>();
+    case 9: return variant_info<CfgDefault, 8>();
+    case 10: return variant_info<Cfg2, 16>();
+    case 11: return variant_info<Cfg2, 8>();
+    default:
+      switch (walk_group_size(n)) {
+        case 4: return variant_info<CfgDefault, 4>();
+        case 8: return variant_info<CfgDefault, 8>();
+        case 16: return variant_info<CfgDefault, 16>();
+        default: return variant_info<CfgDefault>();
+      }
   }
 }
 
@@ -660,18 +761,31 @@ void launch_walk_variant(bh_ctx* c, int v, int n, float theta, float eps, float4
   if (n <= 0) return;
   cudaMemsetAsync(&c->counters->group_next, 0, sizeof(unsigned), c->stream);
   c->launches += 1;
-  launch_quad_variant(c, v, n, theta * theta, eps * eps, acc_out, nullptr, 0.f, nullptr, batch);
+  launch_quad_variant(c, v, n, WalkArgs{theta * theta, eps * eps, 0.f, acc_out, nullptr, nullptr, batch});
 }
+
+namespace {
+template <bool kQuad, bool kSelf>
+void walk_grids_all_groups() {
+  walk_grid<kQuad, kSelf, false, CfgDefault, 32>();
+  walk_grid<kQuad, kSelf, false, CfgDefault, 16>();
+  walk_grid<kQuad, kSelf, false, CfgDefault, 8>();
+  walk_grid<kQuad, kSelf, false, CfgDefault, 4>();
+}
+}  // namespace
 
 // Occupancy queries done once per process, before any stream capture.
 void walk_init() {
-  walk_grid<true, true, false, CfgDefault>();
-  walk_grid<true, false, false, CfgDefault>();
-  walk_grid<false, true, false, CfgDefault>();
-  walk_grid<false, false, false, CfgDefault>();
+  walk_grids_all_groups<true, true>();
+  walk_grids_all_groups<true, false>();
+  walk_grids_all_groups<false, true>();
+  walk_grids_all_groups<false, false>();
   walk_grid<true, false, true, CfgDefault>();
   walk_grid<true, false, false, Cfg1>();
   walk_grid<true, false, false, Cfg2>();
+  walk_grid<true, false, false, Cfg2, 16>();
+  walk_grid<true, false, false, Cfg2, 8>();
+  walk_grid<true, false, false, Cfg2, 4>();
   walk_grid<true, false, false, Cfg3>();
   walk_grid<true, false, false, Cfg4>();
   walk_grid<true, false, false, Cfg5>();
@@ -679,37 +793,23 @@ void walk_init() {
   walk_grid<true, false, false, Cfg7>();
 }
 
-#ifndef BH_LITERAL_MIN_GROUP
-#define BH_LITERAL_MIN_GROUP 4
-#endif
-// smallest group of the literal walk (the app's frame, 4 444 bodies: groups of 8 / 4 / 2 walk in
-// 55.1 / 50.5 / 50.5 us)
-constexpr int kLiteralMinGroup = BH_LITERAL_MIN_GROUP;
-
 void launch_walk(bh_ctx* c, int n, float theta, float eps, int mode, float4* acc_slot, float4* vel_kick,
                  float half_dt, bool batch, float4* vel_copy) {
   if (n <= 0) return;
   cudaMemsetAsync(&c->counters->group_next, 0, sizeof(unsigned), c->stream);
   c->launches += 1;
-  const float theta2 = theta * theta, eps2 = eps * eps;
+  const WalkArgs a{theta * theta, eps * eps, half_dt, acc_slot, vel_kick, vel_copy, batch};
   const bool quad = mode == BH_MULTIPOLE_QUADRUPOLE;
-  const bool self = !(eps2 > 0.f);
-  if (quad) {
-    if (self)
-      launch_walk_t<true, true>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch);
-    else
-      launch_quad_variant(c, c->walk_variant, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch);
-  } else {
-    // the literal walk has no tuned variants: its group size follows N, the largest of 32, 16,
-    // 8 and 4 bodies that still gives at least 1024 groups (about seven warps per SM; the tuned
-    // quadrupole walk picks 8 at 4 444 bodies, 16 at 16 384 and 32 at 2^22)
-    int gsize = 32;
-    while (gsize > kLiteralMinGroup && (n + gsize - 1) / gsize < 1024) gsize /= 2;
-    if (self)
-      launch_walk_t<false, true>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, gsize);
-    else
-      launch_walk_t<false, false>(c, n, theta2, eps2, acc_slot, vel_kick, half_dt, vel_copy, batch, gsize);
-  }
+  const bool self = !(a.eps2 > 0.f);
+  const int group = batch ? c->batch_group : walk_group_size(n);
+  if (quad && !self)
+    launch_quad_variant(c, c->walk_variant, n, a);
+  else if (quad)
+    launch_walk_group<true, true>(c, n, a, group);
+  else if (self)
+    launch_walk_group<false, true>(c, n, a, group);
+  else
+    launch_walk_group<false, false>(c, n, a, group);
 }
 
 }  // namespace bh
@@ -727,7 +827,7 @@ void launch_walk_record(bh_ctx* c, int n, float theta, float eps, float4* acc_sl
   const int grid = min(walk_grid<true, false, true, CfgDefault>(), ((n + 31) / 32) / kWarps + 1);
   k_walk<true, false, true><<<grid, kThreads, 0, c->stream>>>(c->wnode, c->tpos, c->tslot, n, theta * theta,
                                                               eps * eps, acc_slot, vel_kick, half_dt, nullptr,
-                                                              nullptr, 0, 32, c->counters, c->err, tape, tape_count,
+                                                              nullptr, 0, c->counters, c->err, tape, tape_count,
                                                               tape_cap);
 }
 
