@@ -360,7 +360,7 @@ bh_status force_at_current(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
     radix_sort_pairs(c, c->tkey, c->tslot, c->keys[1], c->vals[1], n, c->stream, &ko, &vo);
     launch_gather_tree(c, c->tslot, n, c->pos[c->cur], c->tpos);
     launch_build(c, n, p.leaf_capacity);
-    launch_upsweep(c, n, p.leaf_capacity, BH_MULTIPOLE_QUADRUPOLE);
+    launch_upsweep(c, n, BH_MULTIPOLE_QUADRUPOLE);
     if (rec) {
       cudaMemsetAsync(rec->count, 0, sizeof(unsigned), c->stream);
       launch_walk_record(c, n, (float)p.theta, (float)p.eps, c->acc, nullptr, 0.f, rec->chunks, rec->count,
@@ -397,7 +397,7 @@ bh_status fixed_step(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
     radix_sort_pairs(c, c->tkey, c->tslot, c->keys[1], c->vals[1], n, c->stream, &ko, &vo);
     launch_gather_tree(c, c->tslot, n, c->pos[nx], c->tpos);
     launch_build(c, n, p.leaf_capacity);
-    launch_upsweep(c, n, p.leaf_capacity, BH_MULTIPOLE_QUADRUPOLE);
+    launch_upsweep(c, n, BH_MULTIPOLE_QUADRUPOLE);
     if (rec) {
       cudaMemsetAsync(rec->count, 0, sizeof(unsigned), c->stream);
       launch_walk_record(c, n, (float)p.theta, (float)p.eps, c->acc, c->vel[nx], 0.5f * dt, rec->chunks, rec->count,

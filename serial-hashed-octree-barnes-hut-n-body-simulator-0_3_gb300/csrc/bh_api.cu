@@ -50,7 +50,6 @@ bh_status ensure_nodes(bh_ctx* c, size_t need) {
   dfree(c->nup);
   dfree(c->nchildbyte);
   dfree(c->nparent);
-  dfree(c->narrived);
   dfree(c->hash_keys);
   dfree(c->hash_vals);
   c->hash_cap = 0;
@@ -62,7 +61,6 @@ bh_status ensure_nodes(bh_ctx* c, size_t need) {
   BH_TRY(dalloc(&c->nup, cap));
   BH_TRY(dalloc(&c->nchildbyte, cap));
   BH_TRY(dalloc(&c->nparent, cap));
-  BH_TRY(dalloc(&c->narrived, cap));
   c->node_cap = cap;
   c->tree_valid = false;
   return BH_OK;
@@ -189,7 +187,6 @@ bh_status bh_destroy(bh_ctx* c) {
   dfree(c->nup);
   dfree(c->nchildbyte);
   dfree(c->nparent);
-  dfree(c->narrived);
   dfree(c->lb_level);
   dfree(c->level_bounds);
   dfree(c->level_tile_ctr);
@@ -445,7 +442,7 @@ bh_status bh_build(bh_ctx* c, const double center[3], double edge, int leaf_capa
     bh::launch_set_geom(c, center, edge, center, edge);
     enqueue_tree(c, c->pos[c->cur], n, leaf_capacity, multipole, false);
     bh::launch_build(c, n, leaf_capacity);
-    bh::launch_upsweep(c, n, leaf_capacity, multipole);
+    bh::launch_upsweep(c, n, multipole);
     BH_TRY(last_launch());
     uint32_t e = 0;
     BH_TRY(sync_and_check(c, &e));
@@ -697,7 +694,7 @@ void enqueue_plain_step(bh_ctx* c, const bh_params* prm, const HostIO* io, bool 
   mark(5);
   bh::launch_build(c, n, prm->leaf_capacity);
   mark(6);
-  bh::launch_upsweep(c, n, prm->leaf_capacity, prm->multipole);
+  bh::launch_upsweep(c, n, prm->multipole);
   mark(7);
   float4* vel_copy = io ? io->vel_out_dev : nullptr;
   bh::launch_walk(c, n, (float)prm->theta, (float)prm->eps, prm->multipole, c->acc, c->vel[nx], 0.5f * dt, false,
@@ -1009,7 +1006,7 @@ void enqueue_batch_step(bh_ctx* c, const bh_params& p, const HostIO* io, bool ma
   mark(5);
   bh::launch_build(c, n, p.leaf_capacity, true);
   mark(6);
-  bh::launch_upsweep(c, n, p.leaf_capacity, p.multipole, true);
+  bh::launch_upsweep(c, n, p.multipole, true);
   mark(7);
   float4* vel_copy = io ? io->vel_out_dev : nullptr;
   bh::launch_walk(c, n, (float)p.theta, (float)p.eps, p.multipole, c->acc, c->vel[nx], 0.5f * dt, true, vel_copy);

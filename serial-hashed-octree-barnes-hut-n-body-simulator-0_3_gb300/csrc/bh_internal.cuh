@@ -48,6 +48,7 @@ struct Geom {
   float size_hi, size_lo, frac_hi, frac_lo;
   float tc_hi[3], tc_lo[3];
   float tscale_hi, tscale_lo, tmargin_f;
+  float tedge2;  // root edge squared
 };
 
 // Walk record of one node: 64 bytes, read by the tree walk.
@@ -63,7 +64,7 @@ struct __align__(16) WalkNode {
   int4 link;
 };
 
-// Multipole of one node, kept for the parents during the upsweep (64 bytes). Mass and
+// Multipole of one node or body chunk (64 bytes), at full precision. Mass and
 // centre of mass are float-float pairs (value = hi + lo, about 44 significant bits, from
 // compensated FP32 sums: GB300's FP64 pipe is far too slow for this pass); the quadrupole is
 // FP32. hi is the FP32 rounding of the pair, which is what the walk reads.
@@ -73,8 +74,8 @@ struct __align__(16) NodeUp {
   float com_lo[3];
   float mass_lo;
   float q[6];         // Qxx, Qxy, Qxz, Qyy, Qyz, Qzz about the centre of mass
-  uint32_t min_rank;  // smallest Morton slot among members (literal barycentre)
-  uint32_t pad;
+  uint32_t min_slot;  // chunk records, literal mode: the member with the smallest Morton slot
+  uint32_t min_body;  // and its tree position
 };
 
 // One recorded evaluation buffer of the walk (the adjoint replays these): the group it served
@@ -93,6 +94,7 @@ struct Counters {
   unsigned long long cell_evals;   // warp-wide cell entries evaluated (32 lane slots each)
   unsigned long long point_evals;  // warp-wide point entries evaluated
   unsigned int group_next;  // walk work queue
+  unsigned int node_next;   // upsweep work queue
   unsigned int max_depth;
 };
 
@@ -143,8 +145,7 @@ struct bh_ctx {
   bh::WalkNode* wnode = nullptr;
   bh::NodeUp* nup = nullptr;
   uint8_t* nchildbyte = nullptr;
-  int* nparent = nullptr;      // parent node (-1 for roots), for the upsweep
-  uint32_t* narrived = nullptr;  // upsweep: children finished, per node
+  int* nparent = nullptr;      // parent node (-1 for the root), all-depths build
   uint32_t* lb_level = nullptr;  // look-back words of the level build
   int lb_level_tiles = 0;
   int* level_bounds = nullptr;  // [kLevels + 1] node index where each depth starts
@@ -267,7 +268,7 @@ void launch_treekey(bh_ctx* c, const float4* pos, int n, uint64_t* tkeys, uint32
 void launch_kick_drift(bh_ctx* c, float4* pos, float4* vel, const float4* acc, int n, float dt, int drift);
 void launch_gather_tree(bh_ctx* c, const uint32_t* tslot, int n, const float4* pos, float4* tpos);
 void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch = false);
-void launch_upsweep(bh_ctx* c, int n, int leaf_cap, int mode, bool batch = false);
+void launch_upsweep(bh_ctx* c, int n, int mode, bool batch = false);
 void launch_batch_bounds(bh_ctx* c, const float4* pos, double edge_factor);
 void launch_sys_keys(bh_ctx* c, const uint32_t* vals, int n, uint64_t* k2);
 void launch_gather_tree_keys(bh_ctx* c, const uint32_t* tslot, int n, const float4* pos,

@@ -185,6 +185,7 @@ __device__ __forceinline__ void fill_tree_geom(Geom& g, const double tc[3], doub
   ff_split(g.frac, g.frac_hi, g.frac_lo);
   for (int a = 0; a < 3; ++a) ff_split(tc[a], g.tc_hi[a], g.tc_lo[a]);
   ff_split(g.tscale, g.tscale_hi, g.tscale_lo);
+  g.tedge2 = __double2float_rn(__dmul_rn(tedge, tedge));
   g.tmargin_f = __double2float_rn(g.tmargin);
 }
 
@@ -903,22 +904,17 @@ __global__ __launch_bounds__(kPBThreads) void k_nodes_write(const uint64_t* __re
 // their cells adjacent, so a node's cell ends where its next sibling's starts, and a last
 // child's where its parent's ends (the climb passes only through last children: about 1.3
 // nodes on average). The last child of each parent (the next node has another parent) also
-// counts its siblings from the parent's first child and ORs their digits. The upsweep's arrival
-// counters are zeroed here as well (the parent links it needs are k_nodes_write's), so the
-// all-depths build needs no separate k_upsweep_links.
+// counts its siblings from the parent's first child and ORs their digits.
 __global__ __launch_bounds__(kThreads) void k_nodes_link(const int* __restrict__ level_bounds,
                                                          const uint64_t* __restrict__ nkey,
                                                          const int* __restrict__ nparent, int2* __restrict__ nrange,
                                                          WalkNode* __restrict__ wn, uint8_t* __restrict__ childbyte,
-                                                         uint32_t* __restrict__ arrived,
                                                          const uint32_t* __restrict__ err) {
   if (*err & kErrNodes) return;
   const int m = level_bounds[kLevels];
   const int n = nrange[0].y;
-  if (blockIdx.x == 0 && threadIdx.x == 0) arrived[0] = 0u;
   auto last_child = [&](int j) { return j + 1 >= m || nparent[j + 1] != nparent[j]; };
   for (int j = 1 + blockIdx.x * kThreads + threadIdx.x; j < m; j += gridDim.x * kThreads) {
-    arrived[j] = 0u;
     const bool last = last_child(j);
     int a = j;
     bool up = last;
@@ -958,255 +954,439 @@ __device__ __forceinline__ void quad_add(float q[6], float m, float x, float y, 
   q[5] += fmaf(m3 * z, z, -r2m);
 }
 
-// A child's upsweep record as written by another thread of the same launch: read through L2
-// (an L1 line could hold a stale copy fetched for a neighbouring node).
-__device__ __forceinline__ NodeUp load_nodeup(const NodeUp* p) {
-  const float4* f = reinterpret_cast<const float4*>(p);
-  const float4 a = __ldcg(f), b = __ldcg(f + 1), c = __ldcg(f + 2), d = __ldcg(f + 3);
-  NodeUp u;
-  u.com_hi[0] = a.x;
-  u.com_hi[1] = a.y;
-  u.com_hi[2] = a.z;
-  u.mass_hi = a.w;
-  u.com_lo[0] = b.x;
-  u.com_lo[1] = b.y;
-  u.com_lo[2] = b.z;
-  u.mass_lo = b.w;
-  u.q[0] = c.x;
-  u.q[1] = c.y;
-  u.q[2] = c.z;
-  u.q[3] = c.w;
-  u.q[4] = d.x;
-  u.q[5] = d.y;
-  u.min_rank = __float_as_uint(d.z);
-  u.pad = __float_as_uint(d.w);
-  return u;
+// Upsweep without a climb: every node's multipole straight from its bodies. A node is the range
+// [first, first + count) of the tree order, so its mass and centre of mass are range sums and its
+// quadrupole a second range sum about that centre; no node waits for another, where a bottom-up
+// climb is one L2 round trip and one atomic per level and child. Bound by the dependent float-float
+// sums of each node. Device time of the upsweep, climb -> this (chunk launches included): 4 444
+// bodies (literal) 45 -> 12 us, 16 384 (leaf 1) 41 -> 20, 100 003 (leaf 1) 97 -> 41, 2^22 (leaf 16)
+// 250 -> 204, the ensemble of 4.7e7 bodies 4.5 -> 2.35 ms. Chunk records (k_chunk_moments: the moments of every
+// aligned 64 and 4096 bodies) keep a large node's range to at most 126 bodies, 126 chunks and its
+// supers, which bounds the work at 2^22 bodies, where the visits of a body per level would not.
+//   count <= 16     one thread in systems of more than 65 536 bodies (32 nodes per warp: the
+//                   fewest instructions); below that a team, whose chain of sums is shorter
+//   count <= 1024   a team of 8 lanes (128 without chunk records)
+//   count <= 16384  a warp (1024 without)
+//   larger          the block
+// The block collects the larger nodes of its tile and takes them after the small ones. Nodes are
+// numbered level by level, so the largest come first: the head of the list is dealt node by node to
+// all blocks, the rest in tiles of neighbouring nodes from a queue.
+constexpr int kThreadNode = 16;  // largest node of a thread
+constexpr int kTeam = 8;
+constexpr int kTeamDirect = 128, kTeamNode = 1024;  // largest node of a team without / with chunks
+constexpr int kWarpDirect = 1024, kWarpNode = 16384;
+constexpr int kChunk = 64;    // bodies per chunk record
+constexpr int kSuper = 64;    // chunks per super record
+
+// First moments of a range: mass and sum of mass * position, in float-float.
+struct Moments {
+  FF m, x, y, z;
+  __device__ __forceinline__ void body(float4 p) {
+    m = ff_add(m, {p.w, 0.f});
+    x = ff_add(x, ff_prod(p.x, p.w));
+    y = ff_add(y, ff_prod(p.y, p.w));
+    z = ff_add(z, ff_prod(p.z, p.w));
+  }
+  __device__ __forceinline__ void record(const NodeUp& r) {
+    const FF rm = {r.mass_hi, r.mass_lo};
+    m = ff_add(m, rm);
+    x = ff_add(x, ff_mul({r.com_hi[0], r.com_lo[0]}, rm));
+    y = ff_add(y, ff_mul({r.com_hi[1], r.com_lo[1]}, rm));
+    z = ff_add(z, ff_mul({r.com_hi[2], r.com_lo[2]}, rm));
+  }
+  // sums over lanes that differ in the bits below W; the order of the two operands does not
+  // change an ff_add, so every lane ends with the same pair
+  template <int W>
+  __device__ __forceinline__ void reduce() {
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+      m = ff_add(m, {__shfl_xor_sync(0xffffffffu, m.hi, o), __shfl_xor_sync(0xffffffffu, m.lo, o)});
+      x = ff_add(x, {__shfl_xor_sync(0xffffffffu, x.hi, o), __shfl_xor_sync(0xffffffffu, x.lo, o)});
+      y = ff_add(y, {__shfl_xor_sync(0xffffffffu, y.hi, o), __shfl_xor_sync(0xffffffffu, y.lo, o)});
+      z = ff_add(z, {__shfl_xor_sync(0xffffffffu, z.hi, o), __shfl_xor_sync(0xffffffffu, z.lo, o)});
+    }
+  }
+  __device__ __forceinline__ void centre() {  // sums -> centre of mass
+    if (m.hi == 0.f) return;
+    x = ff_div(x, m);
+    y = ff_div(y, m);
+    z = ff_div(z, m);
+  }
+};
+
+// Quadrupole of a range about a centre, FP32 partial sums.
+struct Quad {
+  float q[6];
+  __device__ __forceinline__ void body(float4 p, const Moments& c) {
+    quad_add(q, p.w, (p.x - c.x.hi) - c.x.lo, (p.y - c.y.hi) - c.y.lo, (p.z - c.z.hi) - c.z.lo);
+  }
+  __device__ __forceinline__ void record(const NodeUp& r, const Moments& c) {
+    quad_add(q, r.mass_hi, (r.com_hi[0] - c.x.hi) + (r.com_lo[0] - c.x.lo),
+             (r.com_hi[1] - c.y.hi) + (r.com_lo[1] - c.y.lo), (r.com_hi[2] - c.z.hi) + (r.com_lo[2] - c.z.lo));
+#pragma unroll
+    for (int k = 0; k < 6; ++k) q[k] += r.q[k];
+  }
+  template <int W>
+  __device__ __forceinline__ void reduce() {
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 6; ++k) q[k] += __shfl_xor_sync(0xffffffffu, q[k], o);
+  }
+};
+
+// Literal barycentre: the member with the smallest Morton slot, as (slot << 32 | tree position).
+template <int W>
+__device__ __forceinline__ unsigned long long min_reduce(unsigned long long v) {
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ unsigned long long first_member(const uint32_t* __restrict__ tslot, int b) {
+  return ((unsigned long long)tslot[b] << 32) | (unsigned)b;
 }
 
-// The multipole of one node at depth d (computeTreeBaryCenters / computeNodeBaryCenters,
-// src/HashedOctree.cpp:721-855, as intended; or the literal pseudo-barycentres). A leaf
-// combines its member bodies, an internal node its children, whose records are complete.
-// kPrefetch (small trees, where the climb's latency is the upsweep's time): an internal node
-// loads all its children's records at once before combining them, one L2 round trip instead of
-// one per child and pass; the arithmetic and its order are the same, so are the results.
-template <bool kPrefetch>
-__device__ void upsweep_node(int node, int d, int mode, const float4* __restrict__ tpos,
-                             const uint32_t* __restrict__ tslot, WalkNode* __restrict__ wn, NodeUp* __restrict__ nf,
-                             const Geom* __restrict__ g, const uint16_t* __restrict__ body_sys) {
-  {
-    const int4 link = wn[node].link;
-    // batched ensembles: the node's system (that of its first body) sets the root edge
-    const double edge = ldexp(body_sys ? g[body_sys[link.z]].tedge : g->tedge, -d);
-    const float s2 = (float)(edge * edge);
-    FF mass = {0.f, 0.f}, com[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-    float q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    uint32_t min_rank = 0xffffffffu;
-    bool single = false;
-    if (link.y == 0) {  // leaf: members are tree-order bodies [link.z, link.z + link.w)
-      if (mode == BH_MULTIPOLE_LITERAL) {
-        int first = link.z;
-        for (int b = link.z; b < link.z + link.w; ++b) {
-          mass = ff_add(mass, {tpos[b].w, 0.f});
-          const uint32_t rk = tslot[b];
-          if (rk < min_rank) {
-            min_rank = rk;
-            first = b;
-          }
-        }
-        const float4 p = tpos[first];
-        com[0] = {p.x, 0.f};
-        com[1] = {p.y, 0.f};
-        com[2] = {p.z, 0.f};
-        single = link.w == 1;
-      } else if (link.w == 1) {
-        const float4 p = tpos[link.z];
-        com[0] = {p.x, 0.f};
-        com[1] = {p.y, 0.f};
-        com[2] = {p.z, 0.f};
-        mass = {p.w, 0.f};
-        min_rank = tslot[link.z];
-        single = true;
-      } else {
-        // members in batches of four: the batch's loads are issued together before the
-        // dependent float-float sums (same summation order as one member at a time)
-        const int end = link.z + link.w;
-        for (int b0 = link.z; b0 < end; b0 += 4) {
-          float4 pb[4];
-          uint32_t rb[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            pb[j] = b0 + j < end ? tpos[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-            rb[j] = b0 + j < end ? tslot[b0 + j] : 0xffffffffu;
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (b0 + j >= end) break;
-            const float4 p = pb[j];
-            mass = ff_add(mass, {p.w, 0.f});
-            com[0] = ff_add(com[0], ff_prod(p.x, p.w));
-            com[1] = ff_add(com[1], ff_prod(p.y, p.w));
-            com[2] = ff_add(com[2], ff_prod(p.z, p.w));
-            min_rank = min(min_rank, rb[j]);
-          }
-        }
-        if (mass.hi != 0.f)
-          for (int a = 0; a < 3; ++a) com[a] = ff_div(com[a], mass);
-        for (int b0 = link.z; b0 < end; b0 += 4) {
-          float4 pb[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) pb[j] = b0 + j < end ? tpos[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (b0 + j >= end) break;
-            const float4 p = pb[j];
-            quad_add(q, p.w, (p.x - com[0].hi) - com[0].lo, (p.y - com[1].hi) - com[1].lo,
-                     (p.z - com[2].hi) - com[2].lo);
-          }
-        }
-      }
-    } else if (kPrefetch) {
-      NodeUp ch[8];
-      int cw[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k < link.y) {
-          ch[k] = load_nodeup(nf + link.x + k);
-          cw[k] = mode == BH_MULTIPOLE_LITERAL ? 0 : wn[link.x + k].link.w;
-        }
-      if (mode == BH_MULTIPOLE_LITERAL) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < link.y) {
-            mass = ff_add(mass, {ch[k].mass_hi, ch[k].mass_lo});
-            if (ch[k].min_rank < min_rank) {
-              min_rank = ch[k].min_rank;
-              for (int a = 0; a < 3; ++a) com[a] = {ch[k].com_hi[a], ch[k].com_lo[a]};
-            }
-          }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < link.y) {
-            const FF m = {ch[k].mass_hi, ch[k].mass_lo};
-            mass = ff_add(mass, m);
-            for (int a = 0; a < 3; ++a) com[a] = ff_add(com[a], ff_mul({ch[k].com_hi[a], ch[k].com_lo[a]}, m));
-            min_rank = min(min_rank, ch[k].min_rank);
-          }
-        if (mass.hi != 0.f)
-          for (int a = 0; a < 3; ++a) com[a] = ff_div(com[a], mass);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < link.y) {
-            quad_add(q, ch[k].mass_hi, (ch[k].com_hi[0] - com[0].hi) + (ch[k].com_lo[0] - com[0].lo),
-                     (ch[k].com_hi[1] - com[1].hi) + (ch[k].com_lo[1] - com[1].lo),
-                     (ch[k].com_hi[2] - com[2].hi) + (ch[k].com_lo[2] - com[2].lo));
-            if (cw[k] > 1)
-              for (int j = 0; j < 6; ++j) q[j] += ch[k].q[j];
-          }
+// One node's records from its sums, 16 bytes for each `part` 0..6.
+__device__ __forceinline__ void write_multipole(int node, int part, const Moments& c, const Quad& q, bool single,
+                                                float s2, WalkNode* __restrict__ wn, NodeUp* __restrict__ nf) {
+  float4 v;
+  switch (part) {
+    case 0: v = make_float4(c.x.hi, c.y.hi, c.z.hi, c.m.hi); break;
+    case 1: v = make_float4(c.x.lo, c.y.lo, c.z.lo, c.m.lo); break;
+    case 2: v = make_float4(q.q[0], q.q[1], q.q[2], q.q[3]); break;
+    case 3: v = make_float4(q.q[4], q.q[5], 0.f, 0.f); break;
+    case 4: v = make_float4(c.x.hi, c.y.hi, c.z.hi, single ? -s2 : s2); break;
+    case 5: v = make_float4(c.m.hi, q.q[0], q.q[1], q.q[2]); break;
+    default: v = make_float4(q.q[3], q.q[4], q.q[5], 0.f); break;
+  }
+  float4* dst = part < 4 ? reinterpret_cast<float4*>(nf + node) + part
+                         : (part == 4 ? &wn[node].mac : (part == 5 ? &wn[node].mq : &wn[node].q2));
+  *dst = v;
+}
+
+// Edge^2 of a node: the root edge squared in FP64 and rounded, times 4^-depth (exact).
+__device__ __forceinline__ float node_edge2(uint64_t key, int first, const Geom* __restrict__ g,
+                                            const uint16_t* __restrict__ body_sys) {
+  const int d = (63 - __clzll((long long)key)) / 3;
+  return ldexpf(body_sys ? g[body_sys[first]].tedge2 : g->tedge2, -2 * d);
+}
+
+// A node's range as bodies, chunks and supers: bodies [first, b0) and [b1, end), chunks [c0, d0)
+// and [d1, c1), supers [s0, s1). Without chunks (or supers) their ranges are empty.
+struct Split {
+  int first, b0, b1, end, c0, d0, d1, c1, s0, s1;
+  __device__ __forceinline__ Split(int2 r, const NodeUp* chunks, const NodeUp* supers) {
+    first = r.x;
+    end = r.x + r.y;
+    b0 = b1 = end;
+    c0 = d0 = d1 = c1 = s0 = s1 = 0;
+    if (!chunks) return;
+    const int lo = (first + kChunk - 1) / kChunk, hi = end / kChunk;
+    if (lo >= hi) return;
+    b0 = lo * kChunk;
+    b1 = hi * kChunk;
+    c0 = lo;
+    d0 = d1 = c1 = hi;
+    const int slo = (lo + kSuper - 1) / kSuper, shi = hi / kSuper;
+    if (!supers || slo >= shi) return;
+    d0 = slo * kSuper;
+    d1 = shi * kSuper;
+    s0 = slo;
+    s1 = shi;
+  }
+  // body(p, b) for every body and record(r) for every record, thread l of W
+  template <class Body, class Record>
+  __device__ __forceinline__ void each(int l, int W, const float4* __restrict__ tpos,
+                                       const NodeUp* __restrict__ chunks, const NodeUp* __restrict__ supers,
+                                       Body body, Record record) const {
+    const int nhead = b0 - first, nbody = nhead + (end - b1);
+#pragma unroll 2
+    for (int i = l; i < nbody; i += W) {
+      const int b = i < nhead ? first + i : b1 + (i - nhead);
+      body(tpos[b], b);
+    }
+    if (c0 >= c1) return;
+    const int chead = d0 - c0, nchunk = chead + (c1 - d1);
+#pragma unroll 2
+    for (int i = l; i < nchunk; i += W) record(chunks[i < chead ? c0 + i : d1 + (i - chead)]);
+#pragma unroll 2
+    for (int i = s0 + l; i < s1; i += W) record(supers[i]);
+  }
+};
+
+// Moments of every aligned kChunk bodies (a team each) or, with records, of every kSuper chunk
+// records (a warp each): mass, centre of mass and quadrupole, or, in literal mode, the mass and the
+// member with the smallest Morton slot.
+template <bool kQuad, int W>
+__global__ __launch_bounds__(kThreads) void k_chunk_moments(const float4* __restrict__ tpos,
+                                                            const uint32_t* __restrict__ tslot,
+                                                            const NodeUp* __restrict__ recs, int n, int per,
+                                                            NodeUp* __restrict__ out) {
+  const int l = threadIdx.x % W, chunk = blockIdx.x * (kThreads / W) + threadIdx.x / W;
+  const long long b0 = (long long)chunk * per, b1 = min((long long)n, b0 + per);
+  Moments c = {};
+  Quad q = {};
+  unsigned long long who = ~0ull;
+  for (long long b = b0 + l; b < b1; b += W) {
+    if (recs) {
+      const NodeUp r = recs[b];
+      if (kQuad)
+        c.record(r);
+      else {
+        c.m = ff_add(c.m, {r.mass_hi, r.mass_lo});
+        who = min(who, ((unsigned long long)r.min_slot << 32) | r.min_body);
       }
     } else {
-      if (mode == BH_MULTIPOLE_LITERAL) {
-        for (int c = link.x; c < link.x + link.y; ++c) {
-          const NodeUp ch = load_nodeup(nf + c);
-          mass = ff_add(mass, {ch.mass_hi, ch.mass_lo});
-          if (ch.min_rank < min_rank) {
-            min_rank = ch.min_rank;
-            for (int a = 0; a < 3; ++a) com[a] = {ch.com_hi[a], ch.com_lo[a]};
-          }
-        }
-      } else {
-        // (batching the children's loads like the leaf members' measured slower here)
-        for (int c = link.x; c < link.x + link.y; ++c) {
-          const NodeUp ch = load_nodeup(nf + c);
-          const FF m = {ch.mass_hi, ch.mass_lo};
-          mass = ff_add(mass, m);
-          for (int a = 0; a < 3; ++a) com[a] = ff_add(com[a], ff_mul({ch.com_hi[a], ch.com_lo[a]}, m));
-          min_rank = min(min_rank, ch.min_rank);
-        }
-        if (mass.hi != 0.f)
-          for (int a = 0; a < 3; ++a) com[a] = ff_div(com[a], mass);
-        for (int c = link.x; c < link.x + link.y; ++c) {
-          const NodeUp ch = load_nodeup(nf + c);
-          quad_add(q, ch.mass_hi, (ch.com_hi[0] - com[0].hi) + (ch.com_lo[0] - com[0].lo),
-                   (ch.com_hi[1] - com[1].hi) + (ch.com_lo[1] - com[1].lo),
-                   (ch.com_hi[2] - com[2].hi) + (ch.com_lo[2] - com[2].lo));
-          if (wn[c].link.w > 1)
-            for (int k = 0; k < 6; ++k) q[k] += ch.q[k];
-        }
+      const float4 p = tpos[b];
+      if (kQuad)
+        c.body(p);
+      else {
+        c.m = ff_add(c.m, {p.w, 0.f});
+        who = min(who, first_member(tslot, (int)b));
       }
     }
-    NodeUp out;
-    for (int a = 0; a < 3; ++a) {
-      out.com_hi[a] = com[a].hi;
-      out.com_lo[a] = com[a].lo;
+  }
+  c.reduce<W>();
+  if (kQuad) {
+    c.centre();
+    for (long long b = b0 + l; b < b1; b += W) {
+      if (recs)
+        q.record(recs[b], c);
+      else
+        q.body(tpos[b], c);
     }
-    out.mass_hi = mass.hi;
-    out.mass_lo = mass.lo;
-    for (int k = 0; k < 6; ++k) out.q[k] = q[k];
-    out.min_rank = min_rank;
-    out.pad = 0;
-    nf[node] = out;
-    wn[node].mac = make_float4(com[0].hi, com[1].hi, com[2].hi, single ? -s2 : s2);
-    wn[node].mq = make_float4(mass.hi, q[0], q[1], q[2]);
-    wn[node].q2 = make_float4(q[3], q[4], q[5], 0.f);
+    q.reduce<W>();
+  } else {
+    who = min_reduce<W>(who);
+  }
+  if (b0 >= n || l != 0) return;
+  NodeUp r;
+  r.com_hi[0] = c.x.hi;
+  r.com_hi[1] = c.y.hi;
+  r.com_hi[2] = c.z.hi;
+  r.com_lo[0] = c.x.lo;
+  r.com_lo[1] = c.y.lo;
+  r.com_lo[2] = c.z.lo;
+  r.mass_hi = c.m.hi;
+  r.mass_lo = c.m.lo;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) r.q[k] = q.q[k];
+  r.min_slot = (uint32_t)(who >> 32);
+  r.min_body = (uint32_t)who;
+  out[chunk] = r;
+}
+
+// A node of one thread, team or warp (W lanes, lane l of it).
+template <bool kQuad, int W>
+__device__ __forceinline__ void node_direct(int node, int2 r, int l, const uint64_t* __restrict__ nkey,
+                                            const float4* __restrict__ tpos, const uint32_t* __restrict__ tslot,
+                                            const NodeUp* __restrict__ chunks, WalkNode* __restrict__ wn,
+                                            NodeUp* __restrict__ nf, const Geom* __restrict__ g,
+                                            const uint16_t* __restrict__ body_sys) {
+  const int end = r.x + r.y;
+  Moments c = {};
+  Quad q = {};
+  if (r.y == 1) {
+    const float4 p = tpos[r.x];
+    c.m = {p.w, 0.f};
+    c.x = {p.x, 0.f};
+    c.y = {p.y, 0.f};
+    c.z = {p.z, 0.f};
+  }
+  const bool many = r.y > 1;
+  if (__any_sync(0xffffffffu, many)) {
+    Moments s = {};
+    unsigned long long who = ~0ull;
+    auto add = [&](float4 p, int b) {
+      if (kQuad)
+        s.body(p);
+      else {
+        s.m = ff_add(s.m, {p.w, 0.f});
+        who = min(who, first_member(tslot, b));
+      }
+    };
+    auto quad = [&](float4 p, int) { q.body(p, s); };
+    // one thread: four bodies' loads together, then the dependent sums
+    auto batches = [&](auto f) {
+      for (int b0 = r.x; b0 < end; b0 += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = tpos[min(b0 + j, end - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (b0 + j < end) f(p[j], b0 + j);
+      }
+    };
+    const Split sp(many ? r : make_int2(0, 0), W > 1 ? chunks : nullptr, nullptr);
+    if (W == 1) {
+      if (many) batches(add);
+    } else {
+      sp.each(l, W, tpos, chunks, nullptr, add, [&](const NodeUp& rec) {
+        if (kQuad)
+          s.record(rec);
+        else {
+          s.m = ff_add(s.m, {rec.mass_hi, rec.mass_lo});
+          who = min(who, ((unsigned long long)rec.min_slot << 32) | rec.min_body);
+        }
+      });
+    }
+    s.reduce<W>();
+    if (kQuad) {
+      s.centre();
+      if (W == 1) {
+        if (many) batches(quad);
+      } else {
+        sp.each(l, W, tpos, chunks, nullptr, quad, [&](const NodeUp& rec) { q.record(rec, s); });
+      }
+      q.reduce<W>();
+    } else {
+      who = min_reduce<W>(who);
+      if (many) {
+        const float4 p = tpos[(uint32_t)who];
+        s.x = {p.x, 0.f};
+        s.y = {p.y, 0.f};
+        s.z = {p.z, 0.f};
+      }
+    }
+    if (many) c = s;
+  }
+  if (r.y <= 0) return;
+  const float s2 = node_edge2(nkey[node], r.x, g, body_sys);
+  if (W > 1) {
+    if (l < 7) write_multipole(node, l, c, q, r.y == 1, s2, wn, nf);
+  } else {
+#pragma unroll
+    for (int part = 0; part < 7; ++part) write_multipole(node, part, c, q, r.y == 1, s2, wn, nf);
   }
 }
 
-// Parent links of the tree just built, and the arrival counters of the upsweep.
-__global__ __launch_bounds__(kThreads) void k_upsweep_links(const int* __restrict__ level_bounds,
-                                                            const WalkNode* __restrict__ wn, int* __restrict__ parent,
-                                                            uint32_t* __restrict__ arrived,
-                                                            const uint32_t* __restrict__ err) {
-  if (*err & kErrNodes) return;
-  const int m = level_bounds[kLevels], roots = level_bounds[1];
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < m; i += gridDim.x * kThreads) {
-    arrived[i] = 0u;
-    if (i < roots) parent[i] = -1;
-    const int4 link = wn[i].link;
-    for (int c = link.x; c < link.x + link.y; ++c) parent[c] = i;
-  }
-}
-
-// The bottom-up multipole pass in one launch. A thread per leaf computes the leaf, then climbs:
-// having published a node, it counts itself in at the parent; the thread
-// that completes the parent's count (the last of the children to finish) computes the parent
-// from all its children, in child order, and goes on up. Every node is computed once, from
-// complete children, with the arithmetic and order of a level-by-level pass, and no thread
-// ever waits for another.
-template <bool kPrefetch>
-__global__ __launch_bounds__(kThreads) void k_upsweep(int mode, const int* __restrict__ level_bounds,
-                                                      const uint64_t* __restrict__ nkey,
-                                                      const int* __restrict__ parent, uint32_t* __restrict__ arrived,
-                                                      const float4* __restrict__ tpos,
-                                                      const uint32_t* __restrict__ tslot,
-                                                      WalkNode* __restrict__ wn, NodeUp* __restrict__ nf,
-                                                      const Geom* __restrict__ g, const uint16_t* __restrict__ body_sys,
-                                                      const uint32_t* __restrict__ err, Counters* __restrict__ ctr) {
+// The multipole of every node (computeTreeBaryCenters / computeNodeBaryCenters,
+// src/HashedOctree.cpp:721-855, as intended; or the literal pseudo-barycentres).
+// kFirst lanes (1 or kTeam) take each node of up to kFirstNode bodies in the first place.
+template <bool kQuad, int kFirst>
+__global__ __launch_bounds__(kThreads) void k_multipoles(const int* __restrict__ level_bounds,
+                                                         const uint64_t* __restrict__ nkey,
+                                                         const int2* __restrict__ nrange,
+                                                         const float4* __restrict__ tpos,
+                                                         const uint32_t* __restrict__ tslot,
+                                                         const NodeUp* __restrict__ chunks,
+                                                         const NodeUp* __restrict__ supers,
+                                                         WalkNode* __restrict__ wn, NodeUp* __restrict__ nf,
+                                                         const Geom* __restrict__ g,
+                                                         const uint16_t* __restrict__ body_sys,
+                                                         const uint32_t* __restrict__ err, Counters* __restrict__ ctr) {
+  constexpr int kWarps = kThreads / 32, kTeams = kThreads / kTeam;
+  constexpr int kNodes = kThreads / kFirst;  // nodes per block and pass
+  __shared__ int s_team[kNodes], s_warp[kNodes], s_big[kNodes];
+  __shared__ int s_count[3], s_next;
+  __shared__ Moments s_mom[kWarps];
+  __shared__ Quad s_quad[kWarps];
+  __shared__ unsigned long long s_who[kWarps];
   if (*err & kErrNodes) return;
   const int m = level_bounds[kLevels];
-  unsigned deepest = 0;
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < m; i += gridDim.x * kThreads) {
-    if (wn[i].link.y != 0) continue;  // internal: computed by its last child's thread
-    int node = i;
-    int d = (63 - __clzll((long long)nkey[i])) / 3;
-    deepest = max(deepest, (unsigned)d);
-    for (;;) {
-      upsweep_node<kPrefetch>(node, d, mode, tpos, tslot, wn, nf, g, body_sys);
-      const int p = parent[node];
-      if (p < 0) break;
-      // the parent's child count (written by the build) can be read before the arrival atomic
-      const int pchildren = kPrefetch ? wn[p].link.y : 0;
-      // acquire-release: this node's stores are visible to the thread that completes the
-      // parent, and that thread sees every child's stores
-      unsigned prev;
-      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(arrived + p) : "memory");
-      if (prev + 1u < (unsigned)(kPrefetch ? pchildren : wn[p].link.y)) break;
-      node = p;
-      --d;
-    }
+  const int team_node = chunks ? kTeamNode : kTeamDirect, warp_node = chunks ? kWarpNode : kWarpDirect;
+  const int first_node = kFirst == 1 ? kThreadNode : team_node;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (blockIdx.x == 0 && t == 0) {
+    int d = 0;
+    while (d < kMaxDepth && level_bounds[d + 2] > level_bounds[d + 1]) ++d;
+    ctr->max_depth = d;
   }
-  deepest = __reduce_max_sync(0xffffffffu, deepest);
-  if ((threadIdx.x & 31) == 0 && deepest > 0) atomicMax(&ctr->max_depth, deepest);
+  if (t < 3) s_count[t] = 0;
+  __syncthreads();
+  // the head: the first nodes of the tree, among them the largest, dealt one by one to the blocks
+  // (a node per warp, or per team in small systems); then tiles of neighbouring nodes from a queue
+  const int head = kFirst == 1 ? kWarps * (int)gridDim.x : kTeams * (int)gridDim.x;
+  for (int tile = -1;;) {
+    int node, l;
+    if (tile < 0 && kFirst == 1) {
+      l = lane;
+      node = lane == 0 ? w * (int)gridDim.x + (int)blockIdx.x : m;
+    } else {
+      l = t % kFirst;
+      node = tile < 0 ? (t / kFirst) * (int)gridDim.x + (int)blockIdx.x : head + tile * kNodes + t / kFirst;
+    }
+    int2 r = node < m ? nrange[node] : make_int2(0, 0);
+    if (r.y > first_node) {
+      if (l == 0) {
+        const int kind = r.y > warp_node ? 2 : (r.y > team_node ? 1 : 0);
+        (kind == 2 ? s_big : (kind == 1 ? s_warp : s_team))[atomicAdd(&s_count[kind], 1)] = node;
+      }
+      r.y = 0;
+    }
+    node_direct<kQuad, kFirst>(node, r, l, nkey, tpos, tslot, chunks, wn, nf, g, body_sys);
+    if (t == 0) s_next = tile < 0 ? (int)blockIdx.x : (int)gridDim.x + (int)atomicAdd(&ctr->node_next, 1u);
+    __syncthreads();
+    tile = s_next;
+    const int nteam = s_count[0], nwarp = s_count[1], nbig = s_count[2];
+    if (kFirst == 1)
+      for (int k = (w * 32) / kTeam; k < nteam; k += kTeams) {  // warp-uniform: a warp takes four nodes
+        const int at = k + lane / kTeam;
+        const int tn = at < nteam ? s_team[at] : 0;
+        node_direct<kQuad, kTeam>(tn, at < nteam ? nrange[tn] : make_int2(0, 0), t % kTeam, nkey, tpos, tslot, chunks, wn,
+                                  nf, g, body_sys);
+      }
+    for (int k = w; k < nwarp; k += kWarps)
+      node_direct<kQuad, 32>(s_warp[k], nrange[s_warp[k]], lane, nkey, tpos, tslot, chunks, wn, nf, g, body_sys);
+    for (int k = 0; k < nbig; ++k) {
+      const int big = s_big[k];
+      const int2 rb = nrange[big];
+      const Split sp(rb, chunks, supers);
+      Moments c = {};
+      Quad q = {};
+      unsigned long long who = ~0ull;
+      sp.each(
+          t, kThreads, tpos, chunks, supers,
+          [&](float4 p, int b) {
+            if (kQuad)
+              c.body(p);
+            else {
+              c.m = ff_add(c.m, {p.w, 0.f});
+              who = min(who, first_member(tslot, b));
+            }
+          },
+          [&](const NodeUp& rec) {
+            if (kQuad)
+              c.record(rec);
+            else {
+              c.m = ff_add(c.m, {rec.mass_hi, rec.mass_lo});
+              who = min(who, ((unsigned long long)rec.min_slot << 32) | rec.min_body);
+            }
+          });
+      c.reduce<32>();
+      if (!kQuad) who = min_reduce<32>(who);
+      if (lane == 0) {
+        s_mom[w] = c;
+        s_who[w] = who;
+      }
+      __syncthreads();
+      c = s_mom[lane % kWarps];
+      c.reduce<kWarps>();
+      if (kQuad) {
+        c.centre();
+        sp.each(
+            t, kThreads, tpos, chunks, supers, [&](float4 p, int) { q.body(p, c); },
+            [&](const NodeUp& rec) { q.record(rec, c); });
+        q.reduce<32>();
+        if (lane == 0) s_quad[w] = q;
+        __syncthreads();
+        q = s_quad[lane % kWarps];
+        q.reduce<kWarps>();
+      } else {
+        who = min_reduce<kWarps>(s_who[lane % kWarps]);
+        const float4 p = tpos[(uint32_t)who];
+        c.x = {p.x, 0.f};
+        c.y = {p.y, 0.f};
+        c.z = {p.z, 0.f};
+      }
+      if (t < 7) write_multipole(big, t, c, q, false, node_edge2(nkey[big], rb.x, g, body_sys), wn, nf);
+      __syncthreads();  // the sums' shared memory serves the next node
+    }
+    __syncthreads();
+    if (t < 3) s_count[t] = 0;
+    __syncthreads();
+    if (head + (long long)tile * kNodes >= m) break;
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1459,8 +1639,8 @@ void launch_gather_tree(bh_ctx* c, const uint32_t* tslot, int n, const float4* p
 // Function attributes set once per process, before any stream capture (none at present).
 void tree_init() {}
 
-// Single trees with leaves of at most kPBMaxLeaf bodies: every depth at once (k_nodes_*), parent
-// links and the upsweep's counters included; otherwise the level build.
+// Single trees with leaves of at most kPBMaxLeaf bodies: every depth at once (k_nodes_*); otherwise
+// the level build.
 bool builds_all_depths(int n, int leaf_cap, bool batch) { return !batch && n >= 1 && leaf_cap <= kPBMaxLeaf; }
 
 void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch) {
@@ -1480,7 +1660,7 @@ void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch) {
                                                         c->level_bounds, (long long)c->node_cap, c->err);
     const int lgrid = (int)std::min<size_t>((size_t)c->sms * 8, (c->node_cap + kThreads - 1) / kThreads);
     k_nodes_link<<<lgrid, kThreads, 0, c->stream>>>(c->level_bounds, c->nkey, c->nparent, c->nrange, c->wnode,
-                                                    c->nchildbyte, c->narrived, c->err);
+                                                    c->nchildbyte, c->err);
     return;
   }
   c->launches += 1 + kLevels;
@@ -1498,34 +1678,46 @@ void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch) {
                                               c->lb_level + (size_t)d * max_tiles, (long long)c->node_cap, c->err);
 }
 
-#ifndef BH_UPSWEEP_PREFETCH_MAX
-#define BH_UPSWEEP_PREFETCH_MAX 65536
-#endif
-// systems of at most this many bodies climb with the children's records prefetched
-constexpr int kUpsweepPrefetchMaxBodies = BH_UPSWEEP_PREFETCH_MAX;
+// Systems above this many bodies sum their larger nodes from chunk records (one more launch, about
+// 6 us: as much as the root's 32 rounds of a block without them),
+constexpr int kChunkMinBodies = 8192;
+// and above this many from super records (another one).
+constexpr int kSuperMinBodies = 262144;
+// Above this many bodies a thread takes each small node, below it a team of kTeam lanes (100 003
+// bodies at leaf capacity 1: 44 us by teams, 35 by threads; 2^22: 415 by teams).
+constexpr int kThreadMinBodies = 65536;
 
-void launch_upsweep(bh_ctx* c, int n, int leaf_cap, int mode, bool batch) {
+void launch_upsweep(bh_ctx* c, int n, int mode, bool batch) {
   if (n <= 0) return;
-  // a thread for every two bodies, about one per node or more at leaf capacity >= 2 (the climbs
-  // want a thread per leaf: at N = 2^22 a fixed 8 blocks per SM took 0.39 ms, this 0.27 ms, the
-  // level-by-level pass it replaces 0.29 ms; at N = 2^25 a fixed 32 blocks per SM took 2.65 ms,
-  // this 1.54 ms)
-  const int grid = std::max(c->sms * 8, (n / 2 + kThreads - 1) / kThreads);
-  // parent links and zeroed arrival counters: written by the all-depths build itself, or here
-  // after the level build
-  if (!builds_all_depths(n, leaf_cap, batch)) {
+  const bool quad = mode == BH_MULTIPOLE_QUADRUPOLE;
+  // the records (about one byte per body) in the sorts' key scratch, free until the next sort
+  NodeUp* chunks = n > kChunkMinBodies ? reinterpret_cast<NodeUp*>(c->keys[1]) : nullptr;
+  NodeUp* supers = nullptr;
+  if (chunks) {
+    const int nchunks = (n + kChunk - 1) / kChunk, teams = kThreads / kTeam;
     c->launches += 1;
-    k_upsweep_links<<<grid, kThreads, 0, c->stream>>>(c->level_bounds, c->wnode, c->nparent, c->narrived, c->err);
+    (quad ? k_chunk_moments<true, kTeam> : k_chunk_moments<false, kTeam>)<<<(nchunks + teams - 1) / teams, kThreads, 0,
+                                                                            c->stream>>>(c->tpos, c->tslot, nullptr, n,
+                                                                                         kChunk, chunks);
+    if (n > kSuperMinBodies) {
+      const int nsupers = (nchunks + kSuper - 1) / kSuper, warps = kThreads / 32;
+      supers = chunks + nchunks;
+      c->launches += 1;
+      (quad ? k_chunk_moments<true, 32> : k_chunk_moments<false, 32>)<<<(nsupers + warps - 1) / warps, kThreads, 0,
+                                                                        c->stream>>>(c->tpos, c->tslot, chunks, nchunks,
+                                                                                     kSuper, supers);
+    }
   }
   c->launches += 1;
-  // the prefetching climb holds eight children's records in registers (one block per SM): two
-  // threads per body there (about one per node at leaf capacity 1), at least a block per SM
-  const bool prefetch = n <= kUpsweepPrefetchMaxBodies;
-  auto upsweep = prefetch ? k_upsweep<true> : k_upsweep<false>;
-  const int ugrid = prefetch ? std::max(c->sms, (2 * n + kThreads - 1) / kThreads) : grid;
-  upsweep<<<ugrid, kThreads, 0, c->stream>>>(mode, c->level_bounds, c->nkey, c->nparent, c->narrived, c->tpos,
-                                              c->tslot, c->wnode, c->nup, batch ? c->sys_geom : c->geom,
-                                              batch ? c->body_sys : nullptr, c->err, c->counters);
+  // up to two nodes per body
+  const bool threads = n > kThreadMinBodies;
+  const int per_pass = kThreads / (threads ? 1 : kTeam);
+  const int grid = (int)std::min<long long>((long long)c->sms * 8, (2ll * n + per_pass - 1) / per_pass);
+  auto kernel = quad ? (threads ? k_multipoles<true, 1> : k_multipoles<true, kTeam>)
+                     : (threads ? k_multipoles<false, 1> : k_multipoles<false, kTeam>);
+  kernel<<<grid, kThreads, 0, c->stream>>>(
+      c->level_bounds, c->nkey, c->nrange, c->tpos, c->tslot, chunks, supers, c->wnode, c->nup,
+      batch ? c->sys_geom : c->geom, batch ? c->body_sys : nullptr, c->err, c->counters);
 }
 
 void launch_batch_bounds(bh_ctx* c, const float4* pos, double edge_factor) {
