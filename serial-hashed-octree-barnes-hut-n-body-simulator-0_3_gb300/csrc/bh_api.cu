@@ -270,8 +270,8 @@ bh_status bh_create(bh_ctx** out, size_t capacity, int device) {
   if (s == BH_OK) s = dalloc(&c->level_bounds, kLevels + 2);
   if (s == BH_OK) s = dalloc(&c->level_tile_ctr, kLevels);
   if (s == BH_OK) s = dalloc(&c->geom, 1);
-  c->bounds_blocks = c->sms * 2;
-  if (s == BH_OK) s = dalloc(&c->bounds_partial, (size_t)c->bounds_blocks * 6);
+  c->bounds_blocks = bh::bounds_blocks(c->sms);
+  if (s == BH_OK) s = dalloc((char**)&c->bounds_partial, bh::bounds_bytes(c->bounds_blocks));
   if (s == BH_OK) s = dalloc(&c->err, 1);
   if (s == BH_OK) s = dalloc(&c->counters, 1);
   if (s != BH_OK) return fail(s);

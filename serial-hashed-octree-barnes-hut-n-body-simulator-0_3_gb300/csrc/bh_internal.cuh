@@ -95,6 +95,7 @@ struct Counters {
   unsigned long long point_evals;  // warp-wide point entries evaluated
   unsigned int group_next;  // walk work queue
   unsigned int node_next;   // upsweep work queue
+  unsigned int bounds_done;  // blocks finished of the bounds kernel
   unsigned int max_depth;
 };
 
@@ -161,7 +162,7 @@ struct bh_ctx {
   double tree_edge = 0;
 
   bh::Geom* geom = nullptr;  // device
-  double* bounds_partial = nullptr;
+  void* bounds_partial = nullptr;  // one partial per block of the bounds kernel
   int bounds_blocks = 0;
   uint32_t* err = nullptr;
   bh::Counters* counters = nullptr;
@@ -255,6 +256,8 @@ void sort_init();
 void walk_init();
 void tree_init();
 
+int bounds_blocks(int sms);
+size_t bounds_bytes(int blocks);
 void launch_bounds(bh_ctx* c, const float4* pos, int n, double edge_factor);
 void launch_set_geom(bh_ctx* c, const double center[3], double size, const double tcenter[3], double tedge);
 void launch_morton(bh_ctx* c, const float4* pos, int n, uint64_t* keys, uint32_t* idx, bool batch = false);

@@ -193,10 +193,84 @@ __device__ __forceinline__ void fill_tree_geom(Geom& g, const double tc[3], doub
 // bounds (OctantBounds(Body*, N), src/OctantUtils.cpp:27-59)
 // ---------------------------------------------------------------------------------------
 
-// Per block: FP64 sums of x, y, z (each thread strides through the bodies in a fixed order,
-// then a fixed-shape tree reduction) and FP32 maxima of |x|, |y|, |z|.
-__global__ __launch_bounds__(kThreads) void k_bounds_partial(const float4* __restrict__ pos, int n,
-                                                             double* __restrict__ partial) {
+// Partial of one block: FP64 sums and FP32 maxima of the absolute coordinates.
+struct BoundsPartial {
+  double sum[3];
+  float mx[3];
+  float pad;
+};
+constexpr int kBoundsPerLane = 10;  // partials per lane of the finishing warp (at most 320 blocks)
+
+// The step's geometry, from the sums and maxima in every lane of one warp: centre = sum * (1 / N)
+// (Vec3D::operator/=, src/MathUtils.cpp:81-90), size = max(0, max_a (max_i |p_ia| - c_a)). fl(|p| - c)
+// is monotone in |p|, so the maximum over bodies of the rounded differences equals the rounded
+// difference of the maximum. The three FP64 quotients run on three lanes at once, and each lane
+// splits one value for the key fast paths (the values are fill_tree_geom's, bit for bit).
+__device__ __forceinline__ void finish_geom(const double (&s)[3], const float (&mx)[3], int n, double inv_n,
+                                            double edge_factor, Geom* __restrict__ g) {
+  const int lane = threadIdx.x & 31;
+  double c[3];
+  double S = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    c[a] = n != 0 ? __dmul_rn(s[a], inv_n) : s[a];
+    const double v = __dsub_rn((double)mx[a], c[a]);
+    if (v > S) S = v;
+  }
+  const double tedge = __dmul_rn(S, edge_factor);
+  const double cm = fmax(fabs(c[0]), fmax(fabs(c[1]), fabs(c[2])));
+  // lane 0: 2^21 / (2 S), lane 1: 2^21 / tedge, lane 2: cm / tedge
+  const double q = __ddiv_rn(lane == 2 ? cm : 2097152.0, lane == 0 ? __dmul_rn(2.0, S) : tedge);
+  // lanes 0-5 hold frac, tscale, margin, size and the centre (6 and 7 its last axes)
+  const double v = lane == 2 ? 0x1p-20 * (1.0 + q) : lane == 3 ? S : lane == 4 ? c[0] : lane == 5 ? c[1] : lane == 6 ? c[2] : q;
+  float hi, lo;
+  ff_split(v, hi, lo);
+  switch (lane) {
+    case 0:
+      g->frac = v;
+      g->frac_hi = hi;
+      g->frac_lo = lo;
+      break;
+    case 1:
+      g->tscale = v;
+      g->tscale_hi = hi;
+      g->tscale_lo = lo;
+      break;
+    case 2:
+      g->tmargin = v;
+      g->tmargin_f = hi;
+      break;
+    case 3:
+      g->size = v;
+      g->size_hi = hi;
+      g->size_lo = lo;
+      break;
+    case 4:
+    case 5:
+    case 6:
+      g->center[lane - 4] = v;
+      g->tc[lane - 4] = v;
+      g->tc_hi[lane - 4] = hi;
+      g->tc_lo[lane - 4] = lo;
+      break;
+    case 7:
+      g->tedge = tedge;
+      g->tedge2 = __double2float_rn(__dmul_rn(tedge, tedge));
+      break;
+    default: break;
+  }
+}
+
+// Bounds in one launch. Per block: FP64 sums of x, y, z (each thread strides through the bodies in a
+// fixed order, then a fixed-shape tree) and FP32 maxima of |x|, |y|, |z|. The last block to finish
+// combines the partials in one warp (lane l sums partials l, l + 32, ... in order, then a fixed
+// shuffle tree): the result does not depend on which block that is. Blocks beyond the bodies
+// would add zeros and are not launched. Bound by FP64 latency (chains of dependent additions on a
+// pipe 64 times slower than FP32): with a second kernel whose finish ran on one lane, a loop of
+// dependent loads and 304 blocks whatever the bodies, the app's frame of 4 444 took 147 us, now 126.
+__global__ __launch_bounds__(kThreads) void k_bounds(const float4* __restrict__ pos, int n, double inv_n,
+                                                     double edge_factor, BoundsPartial* __restrict__ partial,
+                                                     unsigned* __restrict__ done, Geom* __restrict__ g) {
   double sx = 0, sy = 0, sz = 0;
   float mx = 0.f, my = 0.f, mz = 0.f;
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
@@ -208,7 +282,9 @@ __global__ __launch_bounds__(kThreads) void k_bounds_partial(const float4* __res
     my = fmaxf(my, fabsf(p.y));
     mz = fmaxf(mz, fabsf(p.z));
   }
-  __shared__ double sh[6][kThreads / 32];
+  __shared__ double sh[3][kThreads / 32];
+  __shared__ float shm[3][kThreads / 32];
+  __shared__ bool s_last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -223,55 +299,64 @@ __global__ __launch_bounds__(kThreads) void k_bounds_partial(const float4* __res
     sh[0][w] = sx;
     sh[1][w] = sy;
     sh[2][w] = sz;
-    sh[3][w] = mx;
-    sh[4][w] = my;
-    sh[5][w] = mz;
+    shm[0][w] = mx;
+    shm[1][w] = my;
+    shm[2][w] = mz;
   }
   __syncthreads();
-  if (threadIdx.x < 6) {
+  if (threadIdx.x < 3) {
     double acc = sh[threadIdx.x][0];
-    for (int i = 1; i < kThreads / 32; ++i)
-      acc = threadIdx.x < 3 ? __dadd_rn(acc, sh[threadIdx.x][i]) : fmax(acc, sh[threadIdx.x][i]);
-    partial[blockIdx.x * 6 + threadIdx.x] = acc;
-  }
-}
-
-// Combines the partials (one warp: lane l sums partials l, l + 32, ... in order, then a fixed
-// shuffle tree; deterministic, and only ~15 dependent FP64 additions deep): centre = sum *
-// (1 / N) (Vec3D::operator/=, src/MathUtils.cpp:81-90), size = max(0, max_a (max_i |p_ia| -
-// c_a)). fl(|p| - c) is monotone in |p|, so the maximum over bodies of the rounded differences
-// equals the rounded difference of the maximum.
-__global__ void k_bounds_final(const double* __restrict__ partial, int blocks, int n, double edge_factor,
-                               Geom* __restrict__ g) {
-  const int lane = threadIdx.x;
-  double s[3] = {0, 0, 0}, m[3] = {0, 0, 0};
-  for (int b = lane; b < blocks; b += 32)
-    for (int a = 0; a < 3; ++a) {
-      s[a] = __dadd_rn(s[a], partial[b * 6 + a]);
-      m[a] = fmax(m[a], partial[b * 6 + 3 + a]);
+    float m = shm[threadIdx.x][0];
+#pragma unroll
+    for (int i = 1; i < kThreads / 32; ++i) {
+      acc = __dadd_rn(acc, sh[threadIdx.x][i]);
+      m = fmaxf(m, shm[threadIdx.x][i]);
     }
+    partial[blockIdx.x].sum[threadIdx.x] = acc;
+    partial[blockIdx.x].mx[threadIdx.x] = m;
+    __threadfence();
+  }
+  if (w != 0) return;
+  __syncwarp();
+  if (lane == 0) s_last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;  // wraps to 0 for the next launch
+  __syncwarp();
+  if (!s_last) return;
+  __threadfence();
+  double s[3] = {0, 0, 0};
+  float m[3] = {0.f, 0.f, 0.f};
+  double v[kBoundsPerLane][3];
+  float vm[kBoundsPerLane][3];
+#pragma unroll
+  for (int k = 0; k < kBoundsPerLane; ++k) {  // all loads together, then the dependent sums
+    const int b = lane + 32 * k;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      v[k][a] = b < (int)gridDim.x ? __ldcg(&partial[b].sum[a]) : 0.0;
+      vm[k][a] = b < (int)gridDim.x ? __ldcg(&partial[b].mx[a]) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kBoundsPerLane; ++k) {
+    if (32 * k >= (int)gridDim.x) break;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      s[a] = __dadd_rn(s[a], v[k][a]);
+      m[a] = fmaxf(m[a], vm[k][a]);
+    }
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
       s[a] = __dadd_rn(s[a], __shfl_down_sync(0xffffffffu, s[a], o));
-      m[a] = fmax(m[a], __shfl_down_sync(0xffffffffu, m[a], o));
+      m[a] = fmaxf(m[a], __shfl_down_sync(0xffffffffu, m[a], o));
     }
-  if (lane != 0) return;
-  double c[3] = {s[0], s[1], s[2]};
-  double nn = (double)n;
-  if (nn != 0) {
-    double inv = __ddiv_rn(1.0, nn);
-    for (int a = 0; a < 3; ++a) c[a] = __dmul_rn(c[a], inv);
-  }
-  double S = 0;
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    double v = __dsub_rn(m[a], c[a]);
-    if (v > S) S = v;
+    s[a] = __shfl_sync(0xffffffffu, s[a], 0);
+    m[a] = __shfl_sync(0xffffffffu, m[a], 0);
   }
-  for (int a = 0; a < 3; ++a) g->center[a] = c[a];
-  g->size = S;
-  g->frac = __ddiv_rn(2097152.0, __dmul_rn(2.0, S));
-  fill_tree_geom(*g, c, __dmul_rn(S, edge_factor));
+  finish_geom(s, m, n, inv_n, edge_factor, g);
 }
 
 __global__ void k_set_geom(Geom* __restrict__ g, double c0, double c1, double c2, double S, double t0, double t1,
@@ -1471,8 +1556,7 @@ __global__ __launch_bounds__(kThreads) void k_fp32_peak(float* sink, int iters) 
 // ---------------------------------------------------------------------------------------
 
 // OctantBounds of every system, one block per system: FP64 sums in a fixed order (thread
-// stride, then a fixed tree), FP32 maxima of |p|, then the same centre / size / geometry
-// formulas as k_bounds_final.
+// stride, then a fixed tree), FP32 maxima of |p|, then the same finish as k_bounds.
 __global__ __launch_bounds__(kThreads) void k_batch_bounds(const float4* __restrict__ pos,
                                                            const uint32_t* __restrict__ off, double edge_factor,
                                                            Geom* __restrict__ sys_geom) {
@@ -1489,7 +1573,8 @@ __global__ __launch_bounds__(kThreads) void k_batch_bounds(const float4* __restr
     my = fmaxf(my, fabsf(p.y));
     mz = fmaxf(mz, fabsf(p.z));
   }
-  __shared__ double sh[6][kThreads / 32];
+  __shared__ double sh[3][kThreads / 32];
+  __shared__ float shm[3][kThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -1504,36 +1589,25 @@ __global__ __launch_bounds__(kThreads) void k_batch_bounds(const float4* __restr
     sh[0][w] = sx;
     sh[1][w] = sy;
     sh[2][w] = sz;
-    sh[3][w] = mx;
-    sh[4][w] = my;
-    sh[5][w] = mz;
+    shm[0][w] = mx;
+    shm[1][w] = my;
+    shm[2][w] = mz;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  double c[3], m[3];
+  if (w != 0) return;
+  double s3[3];
+  float m3[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    c[a] = sh[a][0];
-    m[a] = sh[3 + a][0];
+    s3[a] = sh[a][0];
+    m3[a] = shm[a][0];
+#pragma unroll
     for (int k = 1; k < kThreads / 32; ++k) {
-      c[a] = __dadd_rn(c[a], sh[a][k]);
-      m[a] = fmax(m[a], sh[3 + a][k]);
+      s3[a] = __dadd_rn(s3[a], sh[a][k]);
+      m3[a] = fmaxf(m3[a], shm[a][k]);
     }
   }
-  const double nn = (double)(b1 - b0);
-  if (nn != 0) {
-    const double inv = __ddiv_rn(1.0, nn);
-    for (int a = 0; a < 3; ++a) c[a] = __dmul_rn(c[a], inv);
-  }
-  double S = 0;
-  for (int a = 0; a < 3; ++a) {
-    const double v = __dsub_rn(m[a], c[a]);
-    if (v > S) S = v;
-  }
-  Geom& g = sys_geom[s];
-  for (int a = 0; a < 3; ++a) g.center[a] = c[a];
-  g.size = S;
-  g.frac = __ddiv_rn(2097152.0, __dmul_rn(2.0, S));
-  fill_tree_geom(g, c, __dmul_rn(S, edge_factor));
+  finish_geom(s3, m3, b1 - b0, __ddiv_rn(1.0, (double)(b1 - b0)), edge_factor, sys_geom + s);
 }
 
 // Secondary sort key: the system of the body each sorted element came from. A stable sort of
@@ -1580,10 +1654,15 @@ inline int grid_for(long long n) { return (int)((n + kThreads - 1) / kThreads); 
 // launchers
 // ---------------------------------------------------------------------------------------
 
+int bounds_blocks(int sms) { return std::min(2 * sms, 32 * kBoundsPerLane); }
+size_t bounds_bytes(int blocks) { return sizeof(BoundsPartial) * (size_t)blocks; }
+
 void launch_bounds(bh_ctx* c, const float4* pos, int n, double edge_factor) {
-  c->launches += 2;
-  k_bounds_partial<<<c->bounds_blocks, kThreads, 0, c->stream>>>(pos, n, c->bounds_partial);
-  k_bounds_final<<<1, 32, 0, c->stream>>>(c->bounds_partial, c->bounds_blocks, n, edge_factor, c->geom);
+  c->launches += 1;
+  const int blocks = std::max(1, std::min(c->bounds_blocks, grid_for(n)));
+  k_bounds<<<blocks, kThreads, 0, c->stream>>>(pos, n, n > 0 ? 1.0 / (double)n : 0.0, edge_factor,
+                                               static_cast<BoundsPartial*>(c->bounds_partial),
+                                               &c->counters->bounds_done, c->geom);
 }
 
 void launch_set_geom(bh_ctx* c, const double center[3], double size, const double tcenter[3], double tedge) {
