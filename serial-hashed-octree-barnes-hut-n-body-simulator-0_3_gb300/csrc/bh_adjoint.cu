@@ -420,7 +420,7 @@ bh_status fixed_step(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
 
 // Copies the tree of the last force evaluation into the tape slot (the chunks are already there).
 bh_status capture_tree(bh_ctx* c, TapeSlot& t) {
-  const int m = c->h_level_bounds[kLevels];
+  const int m = c->h_status->level_bounds[kLevels];
   const int n = (int)c->n;
   if ((size_t)m > t.node_cap) {
     dfree(t.wn);
@@ -577,8 +577,8 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
     }
     BH_TRY(fixed_step(c, a->prm, nullptr));
     if (st) {
-      st->interactions_cell += c->h_counters->cell;
-      st->interactions_p2p += c->h_counters->p2p;
+      st->interactions_cell += c->h_status->counters.cell;
+      st->interactions_p2p += c->h_status->counters.p2p;
     }
   }
   a->final_slot = nck;

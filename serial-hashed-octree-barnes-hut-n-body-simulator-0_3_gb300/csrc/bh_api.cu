@@ -79,20 +79,20 @@ bh_status ensure_hash(bh_ctx* c) {
   return BH_OK;
 }
 
-// Reads the device error word (and the counters) after finishing the stream.
+void copy_status(bh_ctx* c) {
+  cudaMemcpyAsync(c->h_status, c->status, sizeof(bh::Status), cudaMemcpyDeviceToHost, c->stream);
+}
+
 bh_status sync_and_check(bh_ctx* c, uint32_t* err_out) {
-  cudaMemcpyAsync(c->h_err, c->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
-  cudaMemcpyAsync(c->h_counters, c->counters, sizeof(bh::Counters), cudaMemcpyDeviceToHost, c->stream);
-  cudaMemcpyAsync(c->h_level_bounds, c->level_bounds, sizeof(int) * (kLevels + 2), cudaMemcpyDeviceToHost,
-                  c->stream);
+  copy_status(c);
   BH_TRY(cuda_status(cudaStreamSynchronize(c->stream)));
-  if (err_out) *err_out = *c->h_err;
+  if (err_out) *err_out = c->h_status->err;
   return BH_OK;
 }
 
+// The error word and the counters (the walk's and the upsweep's queues among them).
 void clear_device_flags(bh_ctx* c) {
-  cudaMemsetAsync(c->err, 0, sizeof(uint32_t), c->stream);
-  cudaMemsetAsync(c->counters, 0, sizeof(bh::Counters), c->stream);
+  cudaMemsetAsync(c->status, 0, offsetof(bh::Status, level_bounds), c->stream);
 }
 
 size_t initial_node_cap(size_t n) { return std::max<size_t>(2 * n + 64, 1024); }
@@ -179,8 +179,6 @@ bh_status bh_destroy(bh_ctx* c) {
   dfree(c->tslot);
   dfree(c->tpos);
   dfree(c->sort.hist);
-  dfree(c->sort.lookback);
-  dfree(c->sort.tile_ctr);
   dfree(c->nkey);
   dfree(c->nrange);
   dfree(c->wnode);
@@ -188,7 +186,6 @@ bh_status bh_destroy(bh_ctx* c) {
   dfree(c->nchildbyte);
   dfree(c->nparent);
   dfree(c->lb_level);
-  dfree(c->level_bounds);
   dfree(c->level_tile_ctr);
   dfree(c->hash_keys);
   dfree(c->hash_vals);
@@ -204,14 +201,10 @@ bh_status bh_destroy(bh_ctx* c) {
   dfree(c->sys_geom);
   dfree(c->body_sys);
   dfree(c->groups);
-  dfree(c->geom);
   dfree(c->bounds_partial);
-  dfree(c->err);
-  dfree(c->counters);
+  dfree(c->status);
   if (c->flush_buf) cudaFree(c->flush_buf);
-  if (c->h_err) cudaFreeHost(c->h_err);
-  if (c->h_counters) cudaFreeHost(c->h_counters);
-  if (c->h_level_bounds) cudaFreeHost(c->h_level_bounds);
+  if (c->h_status) cudaFreeHost(c->h_status);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
   return BH_OK;
@@ -261,26 +254,27 @@ bh_status bh_create(bh_ctx** out, size_t capacity, int device) {
   if (s == BH_OK) s = dalloc(&c->tslot, capacity);
   if (s == BH_OK) s = dalloc(&c->tpos, capacity);
   c->sort.max_tiles = bh::sort_max_tiles(capacity);
-  if (s == BH_OK) s = dalloc(&c->sort.hist, 8 * 256);
-  if (s == BH_OK) s = dalloc(&c->sort.lookback, (size_t)8 * c->sort.max_tiles * 256);
-  if (s == BH_OK) s = dalloc(&c->sort.tile_ctr, 8);
+  // digit counts, tile counters and look-back words in one block, cleared together by each sort
+  if (s == BH_OK) s = dalloc(&c->sort.hist, 8 * 256 + 8 + (size_t)8 * c->sort.max_tiles * 256);
+  if (s == BH_OK) {
+    c->sort.tile_ctr = c->sort.hist + 8 * 256;
+    c->sort.lookback = c->sort.tile_ctr + 8;
+  }
   // tiles per level: 256 nodes each, or 8 each on the levels built one warp per node
   c->lb_level_tiles = (int)std::max<size_t>((capacity + 255) / 256 + 1, kLevelWarpNodes / 8 + 1);
   if (s == BH_OK) s = dalloc(&c->lb_level, (size_t)kLevels * c->lb_level_tiles);
-  if (s == BH_OK) s = dalloc(&c->level_bounds, kLevels + 2);
   if (s == BH_OK) s = dalloc(&c->level_tile_ctr, kLevels);
-  if (s == BH_OK) s = dalloc(&c->geom, 1);
   c->bounds_blocks = bh::bounds_blocks(c->sms);
   if (s == BH_OK) s = dalloc((char**)&c->bounds_partial, bh::bounds_bytes(c->bounds_blocks));
-  if (s == BH_OK) s = dalloc(&c->err, 1);
-  if (s == BH_OK) s = dalloc(&c->counters, 1);
+  if (s == BH_OK) s = dalloc(&c->status, 1);
   if (s != BH_OK) return fail(s);
-  if (cudaMallocHost((void**)&c->h_err, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_counters, sizeof(bh::Counters)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_level_bounds, sizeof(int) * (kLevels + 2)) != cudaSuccess)
-    return fail(BH_ERR_OOM);
-  cudaMemsetAsync(c->err, 0, sizeof(uint32_t), c->stream);
-  cudaMemsetAsync(c->counters, 0, sizeof(bh::Counters), c->stream);
+  c->counters = &c->status->counters;
+  c->err = &c->status->err;
+  c->level_bounds = c->status->level_bounds;
+  c->geom = &c->status->geom;
+  if (cudaMallocHost((void**)&c->h_status, sizeof(bh::Status)) != cudaSuccess) return fail(BH_ERR_OOM);
+  std::memset(c->h_status, 0, sizeof(bh::Status));
+  cudaMemsetAsync(c->status, 0, sizeof(bh::Status), c->stream);
   cudaMemsetAsync(c->acc, 0, sizeof(float4) * capacity, c->stream);
   cudaMemsetAsync(c->body_key, 0, sizeof(uint64_t) * capacity, c->stream);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(BH_ERR_DEVICE);
@@ -465,7 +459,7 @@ bh_status bh_build(bh_ctx* c, const double center[3], double edge, int leaf_capa
 bh_status bh_tree_size(bh_ctx* c, size_t* m) {
   if (!c || !m) return BH_ERR_INVALID_ARG;
   if (!c->tree_valid) return BH_ERR_NO_TREE;
-  *m = c->n ? (size_t)c->h_level_bounds[kLevels] : 0;
+  *m = c->n ? (size_t)c->h_status->level_bounds[kLevels] : 0;
   return BH_OK;
 }
 
@@ -570,11 +564,11 @@ bh_status bh_force(bh_ctx* c, double theta, double eps, float* acc4_out, bh_stat
     std::memset(st, 0, sizeof(*st));
     st->ms_walk = elapsed(c, 0, 1);
     st->ms_step = st->ms_walk;
-    st->interactions_cell = c->h_counters->cell;
-    st->interactions_p2p = c->h_counters->p2p;
-    st->walk_cell_evals = c->h_counters->cell_evals;
-    st->walk_point_evals = c->h_counters->point_evals;
-    st->n_nodes = (uint64_t)c->h_level_bounds[kLevels];
+    st->interactions_cell = c->h_status->counters.cell;
+    st->interactions_p2p = c->h_status->counters.p2p;
+    st->walk_cell_evals = c->h_status->counters.cell_evals;
+    st->walk_point_evals = c->h_status->counters.point_evals;
+    st->n_nodes = (uint64_t)c->h_status->level_bounds[kLevels];
     st->error_flags = e;
     st->kernel_launches = 1;
   }
@@ -705,6 +699,7 @@ void enqueue_plain_step(bh_ctx* c, const bh_params* prm, const HostIO* io, bool 
       cudaMemcpyAsync(io->vel_out, c->vel[nx], bytes, cudaMemcpyDeviceToHost, c->stream);
     cudaStreamWaitEvent(c->stream, c->io_ev[3], 0);  // join
   }
+  copy_status(c);
 }
 
 bool same_io(const HostIO& a, const void* const b[4]) {
@@ -762,8 +757,8 @@ bh_status run_plain_steps(bh_ctx* c, const bh_params* prm, int nsteps, bh_stats*
       }
       BH_TRY(cuda_status(cudaGraphLaunch(graph, c->stream)));
       c->launches += kernels;
-      BH_TRY(last_launch());
-      BH_TRY(sync_and_check(c, &e));
+      BH_TRY(cuda_status(cudaStreamSynchronize(c->stream)));  // the graph ends with the status copy
+      e = c->h_status->err;
       if (e & bh::kErrNodes) {  // arena too small: grow it (dropping the graphs) and redo the step
         BH_TRY(ensure_nodes(c, c->node_cap * 2));
         if (st) st->retries++;
@@ -790,21 +785,19 @@ bh_status run_plain_steps(bh_ctx* c, const bh_params* prm, int nsteps, bh_stats*
       st->ms_build += elapsed(c, 5, 6);
       st->ms_upsweep += elapsed(c, 6, 7);
       st->ms_walk += elapsed(c, 7, 8);
-      st->n_nodes = (uint64_t)c->h_level_bounds[kLevels];
-      st->interactions_cell += c->h_counters->cell;
-      st->interactions_p2p += c->h_counters->p2p;
-      st->walk_cell_evals += c->h_counters->cell_evals;
-      st->walk_point_evals += c->h_counters->point_evals;
-      st->max_depth = std::max(st->max_depth, c->h_counters->max_depth);
+      st->n_nodes = (uint64_t)c->h_status->level_bounds[kLevels];
+      st->interactions_cell += c->h_status->counters.cell;
+      st->interactions_p2p += c->h_status->counters.p2p;
+      st->walk_cell_evals += c->h_status->counters.cell_evals;
+      st->walk_point_evals += c->h_status->counters.point_evals;
+      st->max_depth = std::max(st->max_depth, c->h_status->counters.max_depth);
       st->steps++;
     }
   }
   if (st) st->kernel_launches = (uint32_t)(c->launches - launches0);
   // tree geometry of the last step, for node lookups
-  bh::Geom g;
-  cudaMemcpy(&g, c->geom, sizeof(g), cudaMemcpyDeviceToHost);
-  for (int a = 0; a < 3; ++a) c->tree_center[a] = g.tc[a];
-  c->tree_edge = g.tedge;
+  for (int a = 0; a < 3; ++a) c->tree_center[a] = c->h_status->geom.tc[a];
+  c->tree_edge = c->h_status->geom.tedge;
   c->hash_valid = false;
   return last_launch();
 }
@@ -1016,6 +1009,7 @@ void enqueue_batch_step(bh_ctx* c, const bh_params& p, const HostIO* io, bool ma
       cudaMemcpyAsync(io->vel_out, c->vel[nx], bytes, cudaMemcpyDeviceToHost, c->stream);
     cudaStreamWaitEvent(c->stream, c->io_ev[3], 0);  // join
   }
+  copy_status(c);
 }
 
 }  // namespace
@@ -1163,7 +1157,8 @@ bh_status run_batch_steps(bh_ctx* c, const bh_params* prm, int nsteps, bh_stats*
       }
       BH_TRY(cuda_status(cudaGraphLaunch(graph, c->stream)));
       c->launches += kernels;
-      BH_TRY(sync_and_check(c, &e));
+      BH_TRY(cuda_status(cudaStreamSynchronize(c->stream)));  // the graph ends with the status copy
+      e = c->h_status->err;
       if (e & bh::kErrNodes) {  // arena too small: grow it, re-capture, redo the step
         destroy_graphs(c);
         BH_TRY(ensure_nodes(c, c->node_cap * 2));
@@ -1184,12 +1179,12 @@ bh_status run_batch_steps(bh_ctx* c, const bh_params* prm, int nsteps, bh_stats*
       st->ms_build += elapsed(c, 5, 6);
       st->ms_upsweep += elapsed(c, 6, 7);
       st->ms_walk += elapsed(c, 7, 8);
-      st->n_nodes = (uint64_t)c->h_level_bounds[kLevels];
-      st->interactions_cell += c->h_counters->cell;
-      st->interactions_p2p += c->h_counters->p2p;
-      st->walk_cell_evals += c->h_counters->cell_evals;
-      st->walk_point_evals += c->h_counters->point_evals;
-      st->max_depth = std::max(st->max_depth, c->h_counters->max_depth);
+      st->n_nodes = (uint64_t)c->h_status->level_bounds[kLevels];
+      st->interactions_cell += c->h_status->counters.cell;
+      st->interactions_p2p += c->h_status->counters.p2p;
+      st->walk_cell_evals += c->h_status->counters.cell_evals;
+      st->walk_point_evals += c->h_status->counters.point_evals;
+      st->max_depth = std::max(st->max_depth, c->h_status->counters.max_depth);
       st->steps++;
     }
   }

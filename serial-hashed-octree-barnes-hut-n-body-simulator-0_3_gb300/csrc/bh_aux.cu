@@ -407,7 +407,7 @@ bh_status bh_tree_boxes(bh_ctx* c, size_t cap, float* center_edge4, int32_t* dep
   if (!c) return BH_ERR_INVALID_ARG;
   if (!c->tree_valid) return BH_ERR_NO_TREE;
   cudaSetDevice(c->device);
-  const size_t m = c->n ? (size_t)c->h_level_bounds[kLevels] : 0;
+  const size_t m = c->n ? (size_t)c->h_status->level_bounds[kLevels] : 0;
   if (cap < m) return BH_ERR_INVALID_ARG;
   if (m == 0) return BH_OK;
   float4* box = nullptr;

@@ -99,6 +99,15 @@ struct Counters {
   unsigned int max_depth;
 };
 
+// The small device results of a context in one block: cleared up to `level_bounds` with one memset at
+// the start of a step and read back whole with one copy at its end.
+struct Status {
+  Counters counters;
+  uint32_t err;
+  int level_bounds[kLevels + 2];
+  Geom geom;
+};
+
 // Radix sort (onesweep) scratch.
 struct SortScratch {
   uint32_t* hist = nullptr;        // [8][256] digit counts, then exclusive offsets
@@ -149,7 +158,7 @@ struct bh_ctx {
   int* nparent = nullptr;      // parent node (-1 for the root), all-depths build
   uint32_t* lb_level = nullptr;  // look-back words of the level build
   int lb_level_tiles = 0;
-  int* level_bounds = nullptr;  // [kLevels + 1] node index where each depth starts
+  int* level_bounds = nullptr;  // [kLevels + 2] node index where each depth starts (in status)
   uint32_t* level_tile_ctr = nullptr;  // [kLevels]
   uint64_t* hash_keys = nullptr;
   int* hash_vals = nullptr;
@@ -161,16 +170,14 @@ struct bh_ctx {
   double tree_center[3] = {0, 0, 0};
   double tree_edge = 0;
 
-  bh::Geom* geom = nullptr;  // device
+  bh::Status* status = nullptr;  // device; geom, err, counters and level_bounds point into it
+  bh::Geom* geom = nullptr;
   void* bounds_partial = nullptr;  // one partial per block of the bounds kernel
   int bounds_blocks = 0;
   uint32_t* err = nullptr;
   bh::Counters* counters = nullptr;
 
-  // host mirror of small device results
-  uint32_t* h_err = nullptr;  // pinned
-  bh::Counters* h_counters = nullptr;
-  int* h_level_bounds = nullptr;
+  bh::Status* h_status = nullptr;  // pinned host mirror, as of the last sync_and_check or step
 
   void* flush_buf = nullptr;
   size_t flush_bytes = 0;
@@ -240,7 +247,9 @@ bh_status cuda_status(cudaError_t e);
 bh_status last_launch();
 bh_status err_to_status(uint32_t e);
 bh_status ensure_nodes(bh_ctx* c, size_t need);
-// Reads the device error word, the counters and the level bounds after finishing the stream.
+// Copies the status block to its host mirror (asynchronous on the context's stream).
+void copy_status(bh_ctx* c);
+// Copies the status block and finishes the stream.
 bh_status sync_and_check(bh_ctx* c, uint32_t* err_out = nullptr);
 void clear_device_flags(bh_ctx* c);
 float elapsed(bh_ctx* c, int a, int b);

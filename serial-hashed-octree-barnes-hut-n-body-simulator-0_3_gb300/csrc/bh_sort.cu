@@ -361,9 +361,9 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);
-  cudaMemsetAsync(c->sort.hist, 0, sizeof(uint32_t) * kPasses * kRadix, st);
-  cudaMemsetAsync(c->sort.lookback, 0, sizeof(uint32_t) * (size_t)kPasses * tiles * kRadix, st);
-  cudaMemsetAsync(c->sort.tile_ctr, 0, sizeof(uint32_t) * kPasses, st);
+  // digit counts, tile counters and look-back words, one block
+  cudaMemsetAsync(c->sort.hist, 0, sizeof(uint32_t) * (kPasses * kRadix + kPasses + (size_t)kPasses * tiles * kRadix),
+                  st);
   int hblocks = (int)min((long long)c->sms * 4, ((long long)n + kThreads * 8 - 1) / (kThreads * 8));
   c->launches += 2 + npasses;
   k_hist<<<hblocks, kThreads, 0, st>>>(keys_in, n, c->sort.hist);

@@ -759,7 +759,6 @@ WalkVariant walk_variant_info(int v, size_t n) {
 // One force-only walk with the given variant (the autotuner's trial); acc_out by slot.
 void launch_walk_variant(bh_ctx* c, int v, int n, float theta, float eps, float4* acc_out, bool batch) {
   if (n <= 0) return;
-  cudaMemsetAsync(&c->counters->group_next, 0, sizeof(unsigned), c->stream);
   c->launches += 1;
   launch_quad_variant(c, v, n, WalkArgs{theta * theta, eps * eps, 0.f, acc_out, nullptr, nullptr, batch});
 }
@@ -796,7 +795,6 @@ void walk_init() {
 void launch_walk(bh_ctx* c, int n, float theta, float eps, int mode, float4* acc_slot, float4* vel_kick,
                  float half_dt, bool batch, float4* vel_copy) {
   if (n <= 0) return;
-  cudaMemsetAsync(&c->counters->group_next, 0, sizeof(unsigned), c->stream);
   c->launches += 1;
   const WalkArgs a{theta * theta, eps * eps, half_dt, acc_slot, vel_kick, vel_copy, batch};
   const bool quad = mode == BH_MULTIPOLE_QUADRUPOLE;
@@ -822,7 +820,6 @@ namespace bh {
 void launch_walk_record(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick, float half_dt,
                         Chunk* tape, unsigned* tape_count, int tape_cap) {
   if (n <= 0) return;
-  cudaMemsetAsync(&c->counters->group_next, 0, sizeof(unsigned), c->stream);
   c->launches += 1;
   const int grid = min(walk_grid<true, false, true, CfgDefault>(), ((n + 31) / 32) / kWarps + 1);
   k_walk<true, false, true><<<grid, kThreads, 0, c->stream>>>(c->wnode, c->tpos, c->tslot, n, theta * theta,
