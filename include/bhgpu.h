@@ -254,14 +254,13 @@ bh_status bh_measure_fp32_peak(bh_ctx* ctx, double* tflops);
  * counterpart in the reference. It is meant for callers that cannot call cudaMalloc where
  * they need the sort: per-frame loops and stream-callback chains, where an allocation or free
  * would synchronise the whole device, and embedders with a fixed device-memory budget. The
- * sort's scratch (ping-pong buffers, histograms, look-back words) lives in a fixed device
- * array of the library, which each GPU holds while the library is loaded, so n is limited to
+ * sort's scratch (the tile-sorted keys and values) lives in a fixed device array of the library,
+ * which each GPU holds while the library is loaded, so n is limited to
  * BH_SORT_STATIC_MAX_KEYS (larger n returns BH_ERR_INVALID_ARG). Sorts stably by the full
  * 64-bit key (the same permutation as bh_sort_bodies) into keys_out / vals_out; the inputs
  * are left unchanged; asynchronous on `stream` (a cudaStream_t, NULL for the legacy default
- * stream) on the current device. status_out (optional, device memory) becomes nonzero if a
- * device-side wait gave up, in which case the output is unspecified; a give-up is reported
- * only there, so a caller that needs to know of one passes status_out.
+ * stream) on the current device. status_out (optional, device memory) is set to 0: the sort's two
+ * launches have no device-side wait that could give up.
  * The first call on each device looks up the scratch array's device address, so make it before
  * any stream capture on that device. The address is kept for the life of the process: after a
  * cudaDeviceReset (which unloads the library's device code) the entry point must not be called

@@ -354,11 +354,7 @@ bh_status force_at_current(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
   for (;;) {
     clear_device_flags(c);
     launch_bounds(c, c->pos[c->cur], n, p.edge_factor);
-    launch_treekey(c, c->pos[c->cur], n, c->tkey, c->tslot);
-    uint64_t* ko;
-    uint32_t* vo;
-    radix_sort_pairs(c, c->tkey, c->tslot, c->keys[1], c->vals[1], n, c->stream, &ko, &vo);
-    launch_gather_tree(c, c->tslot, n, c->pos[c->cur], c->tpos);
+    launch_tree_order(c, c->pos[c->cur], n);
     launch_build(c, n, p.leaf_capacity);
     launch_upsweep(c, n, BH_MULTIPOLE_QUADRUPOLE);
     if (rec) {
@@ -390,12 +386,14 @@ bh_status fixed_step(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
     const int nx = 1 - c->cur;
     clear_device_flags(c);
     launch_bounds(c, c->pos[c->cur], n, p.edge_factor);
-    launch_gather_kd_treekey(c, nullptr, n, c->pos[c->cur], c->vel[c->cur], c->acc, 1, dt, c->pos[nx], c->vel[nx],
-                             c->tkey, c->tslot);
-    uint64_t* ko;
-    uint32_t* vo;
-    radix_sort_pairs(c, c->tkey, c->tslot, c->keys[1], c->vals[1], n, c->stream, &ko, &vo);
-    launch_gather_tree(c, c->tslot, n, c->pos[nx], c->tpos);
+    if (n <= tile_sort_max()) {
+      launch_kd_tiles(c, n, c->pos[c->cur], c->vel[c->cur], c->acc, dt, c->pos[nx], c->vel[nx]);
+      launch_merge_tree(c, c->pos[nx], n);
+    } else {
+      launch_gather_kd_treekey(c, nullptr, n, c->pos[c->cur], c->vel[c->cur], c->acc, 1, dt, c->pos[nx], c->vel[nx],
+                               c->tkey, c->tslot);
+      sort_tree_keys(c, c->pos[nx], n);
+    }
     launch_build(c, n, p.leaf_capacity);
     launch_upsweep(c, n, BH_MULTIPOLE_QUADRUPOLE);
     if (rec) {

@@ -191,6 +191,7 @@ struct bh_ctx {
   int4* groups = nullptr;          // device walk groups: first body, body count, root node, system
   int ngroups = 0;
   int batch_group = 32;            // largest group of the table (32, 16, 8 or 4)
+  bool batch_tiles = false;        // the systems sort in two launches (segments of the tile sort)
   size_t sys_cap = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // captured batched step, by state parity
   bh_params graph_params = {};
@@ -276,6 +277,18 @@ void launch_gather(bh_ctx* c, const uint32_t* perm, int n, const float4* pin, co
 void launch_gather_kd_treekey(bh_ctx* c, const uint32_t* perm, int n, const float4* pin, const float4* vin,
                               const float4* acc, int acc_follows_body, float dt, float4* pout, float4* vout,
                               uint64_t* tkeys, uint32_t* tidx, bool batch = false);
+// Single systems of at most this many bodies sort in two launches (bh_tilesort.cuh).
+int tile_sort_max();
+void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch = false);
+void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
+                     float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch = false);
+void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
+                     float4* vout);
+void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch = false);
+void launch_merge_tree(bh_ctx* c, const float4* pos, int n, bool batch = false);
+void sort_tree_keys(bh_ctx* c, const float4* pos, int n);
+// Tree order (tkey, tslot, tpos) of the given positions, from the geometry in c->geom.
+void launch_tree_order(bh_ctx* c, const float4* pos, int n);
 void launch_treekey(bh_ctx* c, const float4* pos, int n, uint64_t* tkeys, uint32_t* tidx);
 void launch_kick_drift(bh_ctx* c, float4* pos, float4* vel, const float4* acc, int n, float dt, int drift);
 void launch_gather_tree(bh_ctx* c, const uint32_t* tslot, int n, const float4* pos, float4* tpos);

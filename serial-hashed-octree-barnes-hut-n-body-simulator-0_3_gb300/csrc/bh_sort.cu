@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "bh_internal.cuh"
+#include "bh_tilesort.cuh"
 
 namespace bh {
 namespace {
@@ -256,87 +257,34 @@ __global__ __launch_bounds__(kThreads, BH_SORT_MIN_BLOCKS) void k_onesweep(const
 }
 
 // ---------------------------------------------------------------------------------------
-// Small sorts by rank counting. Each key's output position is the number of keys that sort
-// before it: the smaller keys, and the equal keys earlier in the input (which makes the sort
-// stable). A block takes 32 consecutive keys i, one per lane, and its eight warps split each
-// staged tile of keys j into eighths; all lanes of a warp compare their key with the same j (a
-// shared-memory broadcast), and the block adds the eight partial counts. That is n^2
-// comparisons spread over the whole GPU (about 20 M at 4 444 keys), where the eight digit passes
-// of a radix sort are a chain of launches, or of barriers inside one block, that costs far more
-// at this size.
+// Small sorts: tiles and their merge (bh_tilesort.cuh), two launches
 // ---------------------------------------------------------------------------------------
-constexpr int kRankThreads = 256;
-constexpr int kRankParts = kRankThreads / 32;
-#ifndef BH_RANK_TILE
-#define BH_RANK_TILE 4096
-#endif
-// keys j staged per round (8 bytes each): 2048 / 4096 / 5120 give 67.0 / 63.6 / 69.4 us per sort
-// at 16 384 keys and 16.6 / 16.4 / 14.4 us at 4 444
-constexpr int kRankTile = BH_RANK_TILE;
-// Sorts of at most this many keys go by rank: at 4 444 keys 16 us against the radix sort's
-// 68 us, at 16 384 keys 66 us against 74 us (the n^2 comparisons catch up beyond).
-constexpr int kRankSortMax = 16384;
-
-__global__ __launch_bounds__(kThreads) void k_copy_pairs(const uint64_t* __restrict__ kin,
-                                                         const uint32_t* __restrict__ vin,
-                                                         uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                         int n) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i < n) {
-    kout[i] = kin[i];
-    vout[i] = vin[i];
-  }
+__global__ __launch_bounds__(kTileKeys) void k_tile_pairs(const uint64_t* __restrict__ kin,
+                                                          const uint32_t* __restrict__ vin,
+                                                          uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                          int n) {
+  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  tile_sort_store<false>(i < n ? kin[i] : ~0ull, i < n ? vin[i] : 0u, 0u, base, n, kout, vout);
 }
 
-__global__ __launch_bounds__(kRankThreads) void k_sort_rank(const uint64_t* __restrict__ kin,
-                                                            const uint32_t* __restrict__ vin,
-                                                            uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                            int n) {
-  __shared__ uint64_t s_k[kRankTile];
-  __shared__ uint32_t s_cnt[kRankParts][32];
-  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
-  const int base = blockIdx.x * 32, i = base + lane;
-  const bool valid = i < n;
-  const uint64_t ki = valid ? kin[i] : 0ull;
-  uint32_t cnt = 0;
-  // the keys j come through shared memory a tile at a time (one coalesced read of the tile by the
-  // block, instead of a chain of dependent-latency broadcast reads from L2 per warp); warp `part`
-  // compares its lanes' keys with its eighth of the tile
-  for (int t0 = 0; t0 < n; t0 += kRankTile) {
-    const int m = min(kRankTile, n - t0);
-#pragma unroll
-    for (int r = 0; r < kRankTile / kRankThreads; ++r) {
-      const int q = r * kRankThreads + threadIdx.x;
-      if (q < m) s_k[q] = kin[t0 + q];
-    }
-    __syncthreads();
-    const int j0 = t0 + part * (kRankTile / kRankParts);
-    const int j1 = min(t0 + m, j0 + kRankTile / kRankParts);
-    const uint64_t* sk = s_k - t0;  // sk[j] is key j
-    const int below = min(j1, base);  // j before all of this warp's keys: equal keys sort first
-#pragma unroll 8
-    for (int j = j0; j < below; ++j) cnt += sk[j] <= ki ? 1u : 0u;
-    const int d1 = min(j1, base + 32);  // this warp's own keys: equal ones sort first when j < i
-    for (int j = max(j0, base); j < d1; ++j) {
-      const uint64_t kj = sk[j];
-      cnt += (kj < ki || (kj == ki && j < i)) ? 1u : 0u;
-    }
-#pragma unroll 8
-    for (int j = max(j0, base + 32); j < j1; ++j) cnt += sk[j] < ki ? 1u : 0u;  // after: equal keys sort later
-    __syncthreads();
-  }
-  s_cnt[part][lane] = cnt;
-  __syncthreads();
-  if (part == 0 && valid) {
-    uint32_t r = 0;
-#pragma unroll
-    for (int q = 0; q < kRankParts; ++q) r += s_cnt[q][lane];
-    kout[r] = ki;
-    vout[r] = vin[i];
-  }
+__global__ __launch_bounds__(kMergeThreads) void k_merge_pairs(const uint64_t* __restrict__ kin,
+                                                               const uint32_t* __restrict__ vin,
+                                                               uint64_t* __restrict__ kout,
+                                                               uint32_t* __restrict__ vout, int n) {
+  int place;
+  uint64_t key;
+  uint32_t val;
+  if (!tile_merge_rank<false>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
+  kout[place] = key;
+  vout[place] = val;
 }
 
 }  // namespace
+
+// Stages from the keys to the tree order of one step, radix sort / two-launch sort (us, theta 1.2, leaf
+// capacity 8): 1 000 bodies 116 / 36; 4 444 147 / 41; 16 384 155 / 49; 65 536 172 / 88; 98 304 171 / 139;
+// 131 072 176 / 178; 262 144 192 / 512.
+int tile_sort_max() { return 98304; }
 
 int sort_max_tiles(size_t n) { return (int)((n + kTile - 1) / kTile); }
 
@@ -353,11 +301,11 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
   *keys_out = keys_in;
   *vals_out = vals_in;
   if (n <= 1) return;
-  if (n <= kRankSortMax && first_pass == 0 && npasses == kPasses) {
+  if (n <= tile_sort_max() && first_pass == 0 && npasses == kPasses) {
     // the result goes back to keys_in / vals_in, as after the eight digit passes
     c->launches += 2;
-    k_copy_pairs<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(keys_in, vals_in, keys_tmp, vals_tmp, n);
-    k_sort_rank<<<(n + 31) / 32, kRankThreads, 0, st>>>(keys_tmp, vals_tmp, keys_in, vals_in, n);
+    k_tile_pairs<<<tile_blocks(n), kTileKeys, 0, st>>>(keys_in, vals_in, keys_tmp, vals_tmp, n);
+    k_merge_pairs<<<merge_blocks(n), kMergeThreads, 0, st>>>(keys_tmp, vals_tmp, keys_in, vals_in, n);
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);
@@ -396,10 +344,9 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
 // a per-frame loop or a chain of stream callbacks, where cudaMalloc / cudaFree would
 // synchronise the whole device and stall other streams, and embedders that reserve a fixed
 // device-memory budget up front and forbid allocations afterwards. For them this variant keeps
-// every scratch buffer the sort needs (ping-pong key/value buffers, digit histograms, look-back
-// words, tile counters, error word) in one file-scope __device__ array of fixed size, which
-// the GPU holds for as long as the library is loaded. The caller passes only its inputs and
-// outputs.
+// the scratch the sort needs (the tile-sorted keys and values) in one file-scope __device__ array
+// of fixed size, which the GPU holds for as long as the library is loaded. The caller passes only
+// its inputs and outputs.
 //
 // The array's name in host code is only a host-side stand-in for the symbol, not a device
 // address; the device address is resolved with cudaGetSymbolAddress the first time the entry
@@ -412,22 +359,15 @@ namespace bh {
 namespace {
 
 constexpr size_t kStaticMaxKeys = BH_SORT_STATIC_MAX_KEYS;
-constexpr int kStaticTiles = (int)((kStaticMaxKeys + kTile - 1) / kTile);
 constexpr size_t kOffTmpKeys = 0;
 constexpr size_t kOffTmpVals = kOffTmpKeys + kStaticMaxKeys * sizeof(uint64_t);
-constexpr size_t kOffHist = kOffTmpVals + kStaticMaxKeys * sizeof(uint32_t);
-constexpr size_t kOffLookback = kOffHist + (size_t)kPasses * kRadix * sizeof(uint32_t);
-constexpr size_t kOffTileCtr = kOffLookback + (size_t)kPasses * kStaticTiles * kRadix * sizeof(uint32_t);
-constexpr size_t kOffErr = kOffTileCtr + kPasses * sizeof(uint32_t);
-constexpr size_t kStaticBytes = kOffErr + 256;
+constexpr size_t kStaticBytes = kOffTmpVals + kStaticMaxKeys * sizeof(uint32_t);
 
 static __device__ __align__(256) unsigned char g_static_sort_scratch[kStaticBytes];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_static_mutex;
 unsigned char* g_static_addr[kMaxDevices] = {};
-bool g_static_attr[kMaxDevices] = {};
-int g_static_sms[kMaxDevices] = {};
 
 }  // namespace
 }  // namespace bh
@@ -443,7 +383,6 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
     return BH_ERR_DEVICE;
   }
   unsigned char* base = nullptr;
-  int sms = 0;
   {
     std::lock_guard<std::mutex> lock(g_static_mutex);
     if (!g_static_addr[dev]) {
@@ -454,28 +393,11 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
       }
       g_static_addr[dev] = (unsigned char*)p;
     }
-    if (!g_static_attr[dev]) {
-      if (cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(OnesweepSmem)) != cudaSuccess) {
-        cudaGetLastError();
-        return BH_ERR_DEVICE;
-      }
-      g_static_attr[dev] = true;
-    }
-    if (!g_static_sms[dev]) {
-      if (cudaDeviceGetAttribute(&g_static_sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-          g_static_sms[dev] <= 0) {
-        g_static_sms[dev] = 0;
-        cudaGetLastError();
-        return BH_ERR_DEVICE;
-      }
-    }
     base = g_static_addr[dev];
-    sms = g_static_sms[dev];
   }
   cudaStream_t st = (cudaStream_t)stream;
   const int nn = (int)n;
-  if (nn <= 1 && status_out) cudaMemsetAsync(status_out, 0, sizeof(uint32_t), st);
+  if (status_out) cudaMemsetAsync(status_out, 0, sizeof(uint32_t), st);  // this sort waits for nothing
   if (nn == 0) return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ERR_DEVICE;
   if (nn == 1) {
     cudaMemcpyAsync(keys_out, keys_in, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st);
@@ -484,29 +406,7 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
   }
   uint64_t* tmp_keys = (uint64_t*)(base + kOffTmpKeys);
   uint32_t* tmp_vals = (uint32_t*)(base + kOffTmpVals);
-  uint32_t* hist = (uint32_t*)(base + kOffHist);
-  uint32_t* lookback = (uint32_t*)(base + kOffLookback);
-  uint32_t* tile_ctr = (uint32_t*)(base + kOffTileCtr);
-  uint32_t* err = status_out ? status_out : (uint32_t*)(base + kOffErr);
-  const int tiles = sort_max_tiles(n);
-  // everything that must start at zero: histograms, look-back words, tile counters, error word
-  cudaMemsetAsync(hist, 0, kOffErr + sizeof(uint32_t) - kOffHist, st);
-  if (status_out) cudaMemsetAsync(status_out, 0, sizeof(uint32_t), st);
-  const int hblocks = (int)min((long long)sms * 4, ((long long)nn + kThreads * 8 - 1) / (kThreads * 8));
-  k_hist<<<hblocks, kThreads, 0, st>>>(keys_in, nn, hist);
-  k_hist_scan<<<kPasses, kRadix, 0, st>>>(hist);
-  // pass p reads from (p == 0 ? input : buffer of pass p - 1) and writes the tmp buffers on
-  // even passes and the caller's output on odd ones; 8 passes end in the output
-  const uint64_t* ka = keys_in;
-  const uint32_t* va = vals_in;
-  for (int p = 0; p < kPasses; ++p) {
-    uint64_t* kb = (p & 1) ? keys_out : tmp_keys;
-    uint32_t* vb = (p & 1) ? vals_out : tmp_vals;
-    k_onesweep<<<tiles, kThreads, sizeof(OnesweepSmem), st>>>(ka, va, kb, vb, nn, 8 * p, hist + p * kRadix,
-                                                              lookback + (size_t)p * tiles * kRadix,
-                                                              tile_ctr + p, err);
-    ka = kb;
-    va = vb;
-  }
+  k_tile_pairs<<<tile_blocks(nn), kTileKeys, 0, st>>>(keys_in, vals_in, tmp_keys, tmp_vals, nn);
+  k_merge_pairs<<<merge_blocks(nn), kMergeThreads, 0, st>>>(tmp_keys, tmp_vals, keys_out, vals_out, nn);
   return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ERR_DEVICE;
 }

@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "bh_internal.cuh"
+#include "bh_tilesort.cuh"
 
 namespace bh {
 namespace {
@@ -423,9 +424,18 @@ __global__ __launch_bounds__(kThreads) void k_gather(const uint32_t* __restrict_
   vout[j] = vin[i];
 }
 
-// Gather into the new (Morton) order fused with the first half-kick and the drift
-// (ComputePositionAtHalfTimeStep, src/Body.hpp:306-313) and with the tree key of the drifted
-// position.
+// First half-kick and drift of one body (ComputePositionAtHalfTimeStep, src/Body.hpp:306-313).
+__device__ __forceinline__ void kick_drift(float4& p, float4& v, float4 a, float dt, float half_dt) {
+  v.x += a.x * half_dt;
+  v.y += a.y * half_dt;
+  v.z += a.z * half_dt;
+  p.x += v.x * dt;
+  p.y += v.y * dt;
+  p.z += v.z * dt;
+}
+
+// Gather into the new (Morton) order fused with the first half-kick and the drift and with the tree
+// key of the drifted position.
 __global__ __launch_bounds__(kThreads) void k_gather_kd_treekey(
     const uint32_t* __restrict__ perm, int n, const float4* __restrict__ pin, const float4* __restrict__ vin,
     const float4* __restrict__ acc, int acc_follows_body, float dt, float half_dt, const Geom* __restrict__ g,
@@ -434,18 +444,99 @@ __global__ __launch_bounds__(kThreads) void k_gather_kd_treekey(
   int j = blockIdx.x * kThreads + threadIdx.x;
   if (j >= n) return;
   const uint32_t i = perm ? perm[j] : (uint32_t)j;  // no permutation: bodies keep their order
-  float4 p = pin[i], v = vin[i], a = acc[acc_follows_body ? i : (uint32_t)j];
-  v.x += a.x * half_dt;
-  v.y += a.y * half_dt;
-  v.z += a.z * half_dt;
-  p.x += v.x * dt;
-  p.y += v.y * dt;
-  p.z += v.z * dt;
+  float4 p = pin[i], v = vin[i];
+  kick_drift(p, v, acc[acc_follows_body ? i : (uint32_t)j], dt, half_dt);
   pout[j] = p;
   vout[j] = v;
   // the sort keeps every system in its body range, so slot j's system is body_sys[j]
   tkeys[j] = tree_key(p, body_sys ? g[body_sys[j]] : *g);
   tidx[j] = (uint32_t)j;
+}
+
+// ---- systems small enough for the two-launch sort (tile_sort_max): the stages around it in its kernels
+
+// Morton keys, tile-sorted with their slots (kSeg: by the slots' systems first).
+template <bool kSeg>
+__global__ __launch_bounds__(kTileKeys) void k_morton_tiles(const float4* __restrict__ pos, int n,
+                                                            const Geom* __restrict__ g,
+                                                            const uint16_t* __restrict__ body_sys,
+                                                            uint64_t* __restrict__ kout, uint32_t* __restrict__ vout) {
+  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  const uint32_t sys = kSeg ? (i < n ? (uint32_t)body_sys[i] : 0xffffffffu) : 0u;
+  const uint64_t key = i < n ? morton_key(pos[i], kSeg ? g[sys] : *g) : ~0ull;
+  tile_sort_store<kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
+}
+
+// The Morton merge, with k_gather_kd_treekey's work at each body's place in the sorted order: kout
+// (optional) receives the sorted keys, ktree the tree keys by slot.
+template <bool kSeg>
+__global__ __launch_bounds__(kMergeThreads) void k_merge_kd(
+    const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, int n, const float4* __restrict__ pin,
+    const float4* __restrict__ velin, const float4* __restrict__ acc, int acc_follows_body, float dt, float half_dt,
+    const Geom* __restrict__ g, const uint16_t* __restrict__ body_sys, const uint32_t* __restrict__ off,
+    float4* __restrict__ pout, float4* __restrict__ vout, uint64_t* __restrict__ kout, uint64_t* __restrict__ ktree) {
+  int j;
+  uint64_t key;
+  uint32_t i;
+  if (!tile_merge_rank<kSeg>(kin, vin, body_sys, off, n, j, key, i)) return;
+  float4 p = pin[i], v = velin[i];
+  kick_drift(p, v, acc[acc_follows_body ? i : (uint32_t)j], dt, half_dt);
+  pout[j] = p;
+  vout[j] = v;
+  if (kout) kout[j] = key;
+  ktree[j] = tree_key(p, kSeg ? g[body_sys[j]] : *g);
+}
+
+// Tree keys (given, or of the positions), tile-sorted with their slots.
+template <bool kSeg>
+__global__ __launch_bounds__(kTileKeys) void k_tree_tiles(const uint64_t* __restrict__ ktree,
+                                                          const float4* __restrict__ pos, int n,
+                                                          const Geom* __restrict__ g,
+                                                          const uint16_t* __restrict__ body_sys,
+                                                          uint64_t* __restrict__ kout, uint32_t* __restrict__ vout) {
+  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  const uint32_t sys = kSeg ? (i < n ? (uint32_t)body_sys[i] : 0xffffffffu) : 0u;
+  const uint64_t key = i < n ? (ktree ? ktree[i] : tree_key(pos[i], *g)) : ~0ull;
+  tile_sort_store<kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
+}
+
+// The half-kick and drift in place of order (the differentiable path), with the tree keys of the
+// drifted positions tile-sorted.
+__global__ __launch_bounds__(kTileKeys) void k_kd_tiles(const float4* __restrict__ pin,
+                                                        const float4* __restrict__ velin,
+                                                        const float4* __restrict__ acc, int n, float dt, float half_dt,
+                                                        const Geom* __restrict__ g, float4* __restrict__ pout,
+                                                        float4* __restrict__ velout, uint64_t* __restrict__ kout,
+                                                        uint32_t* __restrict__ vout) {
+  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  uint64_t key = ~0ull;
+  if (i < n) {
+    float4 p = pin[i], v = velin[i];
+    kick_drift(p, v, acc[i], dt, half_dt);
+    pout[i] = p;
+    velout[i] = v;
+    key = tree_key(p, *g);
+  }
+  tile_sort_store<false>(key, (uint32_t)i, 0u, base, n, kout, vout);
+}
+
+// The tree-key merge, with the positions gathered into tree order.
+template <bool kSeg>
+__global__ __launch_bounds__(kMergeThreads) void k_merge_tree(const uint64_t* __restrict__ kin,
+                                                              const uint32_t* __restrict__ vin, int n,
+                                                              const float4* __restrict__ pos,
+                                                              const uint16_t* __restrict__ body_sys,
+                                                              const uint32_t* __restrict__ off,
+                                                              uint64_t* __restrict__ tkey,
+                                                              uint32_t* __restrict__ tslot,
+                                                              float4* __restrict__ tpos) {
+  int r;
+  uint64_t key;
+  uint32_t slot;
+  if (!tile_merge_rank<kSeg>(kin, vin, body_sys, off, n, r, key, slot)) return;
+  tkey[r] = key;
+  tslot[r] = slot;
+  tpos[r] = pos[slot];
 }
 
 __global__ __launch_bounds__(kThreads) void k_kick_drift(float4* __restrict__ pos, float4* __restrict__ vel,
@@ -1703,6 +1794,41 @@ void launch_gather_kd_treekey(bh_ctx* c, const uint32_t* perm, int n, const floa
     k_gather_kd_treekey<<<grid_for(n), kThreads, 0, c->stream>>>(
         perm, n, pin, vin, acc, acc_follows_body, dt, 0.5f * dt, batch ? c->sys_geom : c->geom,
         batch ? c->body_sys : nullptr, pout, vout, tkeys, tidx);
+}
+
+// The stages of a step up to the tree order, for systems that sort in two launches. The tile-sorted
+// pairs pass through keys[1] / vals[1].
+void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch) {
+  c->launches += 1;
+  (batch ? k_morton_tiles<true> : k_morton_tiles<false>)<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(
+      pos, n, batch ? c->sys_geom : c->geom, c->body_sys, c->keys[1], c->vals[1]);
+}
+
+void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
+                     float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch) {
+  c->launches += 1;
+  (batch ? k_merge_kd<true> : k_merge_kd<false>)<<<merge_blocks(n), kMergeThreads, 0, c->stream>>>(
+      c->keys[1], c->vals[1], n, pin, vin, acc, acc_follows_body, dt, 0.5f * dt, batch ? c->sys_geom : c->geom,
+      c->body_sys, c->sys_off, pout, vout, kout, ktree);
+}
+
+void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
+                     float4* vout) {
+  c->launches += 1;
+  k_kd_tiles<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(pin, vin, acc, n, dt, 0.5f * dt, c->geom, pout, vout,
+                                                          c->keys[1], c->vals[1]);
+}
+
+void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch) {
+  c->launches += 1;
+  (batch ? k_tree_tiles<true> : k_tree_tiles<false>)<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(
+      ktree, pos, n, c->geom, c->body_sys, c->keys[1], c->vals[1]);
+}
+
+void launch_merge_tree(bh_ctx* c, const float4* pos, int n, bool batch) {
+  c->launches += 1;
+  (batch ? k_merge_tree<true> : k_merge_tree<false>)<<<merge_blocks(n), kMergeThreads, 0, c->stream>>>(
+      c->keys[1], c->vals[1], n, pos, c->body_sys, c->sys_off, c->tkey, c->tslot, c->tpos);
 }
 
 void launch_kick_drift(bh_ctx* c, float4* pos, float4* vel, const float4* acc, int n, float dt, int drift) {
