@@ -572,8 +572,8 @@ __global__ __launch_bounds__(kThreads) void k_gather_tree(const uint32_t* __rest
 // The node set equals the reference's insertion result: the root, plus every prefix K of a
 // body's depth-21 path whose parent holds more than leaf_cap bodies (for leaf capacity 1:
 // count(parent) >= 2). Bodies are sorted by path, so every node is a contiguous body range.
-// Two builds produce the same records: the all-depths build further down (single systems with
-// leaf capacity up to 64), and this level build (ensembles, larger leaf capacities).
+// Two builds produce the same records: the all-depths build further down (leaf capacities up to
+// 64), and this level build (larger ones).
 // One launch per depth turns the internal nodes of depth d into the node records of depth
 // d+1, appended in key order: children get contiguous indices, depths are stored level by
 // level (breadth-first), and a decoupled look-back over 256-node tiles assigns the indices.
@@ -916,28 +916,35 @@ __device__ __forceinline__ void warp_start_counts(int lo, int hi, uint32_t (*s_w
 }
 
 // Start depths of the tile's bodies: lo | hi << 8 (none when lo > hi), and per-warp counts of
-// starts for each depth 1..21 in s_wc.
-__device__ void node_start_depths(const uint64_t* __restrict__ tkey, int n, int leaf_cap, int t0,
-                                  uint32_t (*s_wc)[kPBWarps], uint32_t* span_out) {
+// starts for each depth 1..21 in s_wc. In an ensemble (kSeg) bodies of different systems share no
+// digit, not even the root.
+template <bool kSeg>
+__device__ void node_start_depths(const uint64_t* __restrict__ tkey, const uint16_t* __restrict__ body_sys, int n,
+                                  int leaf_cap, int t0, uint32_t (*s_wc)[kPBWarps], uint32_t* span_out) {
   __shared__ uint64_t s_k[kPBThreads + 2 * kPBMaxLeaf];
+  __shared__ uint16_t s_sys[kSeg ? kPBThreads + 2 * kPBMaxLeaf : 1];
   __shared__ int8_t s_w[kPBThreads + kPBMaxLeaf];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, L = leaf_cap;
+  const int t = threadIdx.x, L = leaf_cap;
   const int base = t0 - L;  // s_k[x - base] is key x, for x in [t0 - L, t0 + T + L)
   for (int x = t; x < kPBThreads + 2 * L; x += kPBThreads) {
     const int g = base + x;
-    s_k[x] = (g >= 0 && g < n) ? tkey[g] : 0ull;
+    const bool in = g >= 0 && g < n;
+    s_k[x] = in ? tkey[g] : 0ull;
+    if (kSeg) s_sys[x] = in ? body_sys[g] : 0;
   }
   __syncthreads();
+  auto shared_digits = [&](int x, int y) {
+    return kSeg && s_sys[x] != s_sys[y] ? -1 : common_digits(s_k[x], s_k[y]);
+  };
   for (int x = t; x < kPBThreads + L; x += kPBThreads) {  // w(j) for j in [t0 - L, t0 + T)
     const int j = base + x;
-    s_w[x] = (int8_t)((j >= 0 && j + L < n) ? common_digits(s_k[x], s_k[x + L]) : -1);
+    s_w[x] = (int8_t)((j >= 0 && j + L < n) ? shared_digits(x, x + L) : -1);
   }
   __syncthreads();
   const int i = t0 + t;
   int lo = 1, hi = 0;
   if (i < n) {
-    const uint64_t ki = s_k[i - base];
-    const int lcp = i == 0 ? -1 : common_digits(s_k[i - 1 - base], ki);
+    const int lcp = i == 0 ? -1 : shared_digits(i - 1 - base, i - base);
     int e = -1;
     for (int q = 0; q <= L; ++q) e = max(e, (int)s_w[t + q]);  // j = i - L + q
     lo = max(lcp + 1, 1);
@@ -948,11 +955,13 @@ __device__ void node_start_depths(const uint64_t* __restrict__ tkey, int n, int 
   __syncthreads();
 }
 
-__global__ __launch_bounds__(kPBThreads) void k_nodes_count(const uint64_t* __restrict__ tkey, int n, int leaf_cap,
+template <bool kSeg>
+__global__ __launch_bounds__(kPBThreads) void k_nodes_count(const uint64_t* __restrict__ tkey,
+                                                            const uint16_t* __restrict__ body_sys, int n, int leaf_cap,
                                                             uint32_t* __restrict__ span,
                                                             uint32_t* __restrict__ tile_cnt, int ntiles) {
   __shared__ uint32_t s_wc[kMaxDepth][kPBWarps];
-  node_start_depths(tkey, n, leaf_cap, blockIdx.x * kPBThreads, s_wc, span);
+  node_start_depths<kSeg>(tkey, body_sys, n, leaf_cap, blockIdx.x * kPBThreads, s_wc, span);
   if (threadIdx.x < kMaxDepth) {
     uint32_t c = 0;
     for (int q = 0; q < kPBWarps; ++q) c += s_wc[threadIdx.x][q];
@@ -999,13 +1008,13 @@ __global__ __launch_bounds__(1024) void k_nodes_scan(uint32_t* __restrict__ tile
 
 // Level starts (s_lb, from the depth totals) and, per depth and warp of this tile, the index of
 // the warp's first node start (s_first); returns the node count.
-__device__ long long node_first_indices(int n, uint32_t lo, uint32_t hi, const uint32_t* __restrict__ tile_excl,
+__device__ long long node_first_indices(int roots, uint32_t lo, uint32_t hi, const uint32_t* __restrict__ tile_excl,
                                         int ntiles, const uint32_t* __restrict__ totals, long long* s_lb,
                                         uint32_t (*s_first)[kPBWarps]) {
   const int t = threadIdx.x;
   if (t == 0) {
     s_lb[0] = 0;
-    s_lb[1] = n > 0 ? 1 : 0;
+    s_lb[1] = roots;
     for (int d = 1; d <= kMaxDepth; ++d) s_lb[d + 1] = s_lb[d] + totals[d - 1];
   }
   warp_start_counts((int)lo, (int)hi, s_first);
@@ -1024,8 +1033,12 @@ __device__ long long node_first_indices(int n, uint32_t lo, uint32_t hi, const u
 
 // Node records from the thread of each node's first body: key, first body, parent, first
 // child (node (d + 1, i); a node is internal exactly when d < the body's deepest start depth).
-// The body counts, child counts and child bytes follow in k_nodes_link.
-__global__ __launch_bounds__(kPBThreads) void k_nodes_write(const uint64_t* __restrict__ tkey, int n, int leaf_cap,
+// The body counts, child counts and child bytes follow in k_nodes_link. The roots come first, one
+// per system of an ensemble (kSeg), from the thread of the system's first body.
+template <bool kSeg>
+__global__ __launch_bounds__(kPBThreads) void k_nodes_write(const uint64_t* __restrict__ tkey,
+                                                            const uint16_t* __restrict__ body_sys,
+                                                            const uint32_t* __restrict__ off, int roots, int n,
                                                             const uint32_t* __restrict__ span,
                                                             const uint32_t* __restrict__ tile_excl, int ntiles,
                                                             const uint32_t* __restrict__ totals,
@@ -1039,7 +1052,7 @@ __global__ __launch_bounds__(kPBThreads) void k_nodes_write(const uint64_t* __re
   const int i = blockIdx.x * kPBThreads + t;
   const uint32_t sp = i < n ? span[i] : 1u;
   const int lo = (int)(sp & 0xFFu), hi = (int)(sp >> 8);
-  const long long m = node_first_indices(n, (uint32_t)lo, (uint32_t)hi, tile_excl, ntiles, totals, s_lb, s_first);
+  const long long m = node_first_indices(roots, (uint32_t)lo, (uint32_t)hi, tile_excl, ntiles, totals, s_lb, s_first);
   if (blockIdx.x == 0) {
     if (t <= kLevels + 1) level_bounds[t] = (int)min(s_lb[min(t, kLevels)], 0x7fffffffll);
     if (t == 0 && m > node_cap) atomicOr(err, kErrNodes);
@@ -1065,14 +1078,16 @@ __global__ __launch_bounds__(kPBThreads) void k_nodes_write(const uint64_t* __re
       child = -1;
     }
   }
-  if (child >= 0) nparent[child] = 0;  // depth-1 nodes hang from the root
-  if (i == 0) {
-    const bool internal = n > leaf_cap;
-    nkey[0] = 1ull;
-    nrange[0] = make_int2(0, n);
-    wn[0].link = make_int4(internal ? 1 : -1, 0, 0, n);
-    childbyte[0] = 0;
-    nparent[0] = -1;
+  if (i >= n) return;
+  const int root = kSeg ? body_sys[i] : 0, first = kSeg ? (int)off[root] : 0;
+  if (child >= 0) nparent[child] = root;  // depth-1 nodes hang from the root
+  if (i == first) {
+    const int count = kSeg ? (int)off[root + 1] - first : n;
+    nkey[root] = 1ull;
+    nrange[root] = make_int2(first, count);
+    wn[root].link = make_int4(child, 0, first, count);  // child: the first depth-1 node, or -1
+    childbyte[root] = 0;
+    nparent[root] = -1;
   }
 }
 
@@ -1087,20 +1102,19 @@ __global__ __launch_bounds__(kThreads) void k_nodes_link(const int* __restrict__
                                                          WalkNode* __restrict__ wn, uint8_t* __restrict__ childbyte,
                                                          const uint32_t* __restrict__ err) {
   if (*err & kErrNodes) return;
-  const int m = level_bounds[kLevels];
-  const int n = nrange[0].y;
+  const int m = level_bounds[kLevels], roots = level_bounds[1];
   auto last_child = [&](int j) { return j + 1 >= m || nparent[j + 1] != nparent[j]; };
-  for (int j = 1 + blockIdx.x * kThreads + threadIdx.x; j < m; j += gridDim.x * kThreads) {
+  for (int j = roots + blockIdx.x * kThreads + threadIdx.x; j < m; j += gridDim.x * kThreads) {
     const bool last = last_child(j);
     int a = j;
     bool up = last;
     while (up) {
       a = nparent[a];
-      if (a == 0) break;
+      if (a < roots) break;
       up = last_child(a);
     }
     const int first = nrange[j].x;
-    const int cnt = (up ? n : nrange[a + 1].x) - first;  // up: the climb reached the root
+    const int cnt = (up ? nrange[a].x + nrange[a].y : nrange[a + 1].x) - first;  // up: the climb reached a root
     nrange[j].y = cnt;
     wn[j].link.w = cnt;
     if (!last) continue;
@@ -1844,12 +1858,8 @@ void launch_gather_tree(bh_ctx* c, const uint32_t* tslot, int n, const float4* p
 // Function attributes set once per process, before any stream capture (none at present).
 void tree_init() {}
 
-// Single trees with leaves of at most kPBMaxLeaf bodies: every depth at once (k_nodes_*); otherwise
-// the level build.
-bool builds_all_depths(int n, int leaf_cap, bool batch) { return !batch && n >= 1 && leaf_cap <= kPBMaxLeaf; }
-
 void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch) {
-  if (builds_all_depths(n, leaf_cap, batch)) {
+  if (n >= 1 && leaf_cap <= kPBMaxLeaf) {
     // every depth at once: counts per tile and depth (in lb_level), their scans (totals in
     // level_tile_ctr), the node records (start depths of each body in vals[1], free after the
     // sorts), then child counts and bytes
@@ -1858,11 +1868,12 @@ void launch_build(bh_ctx* c, int n, int leaf_cap, bool batch) {
     uint32_t* tile = c->lb_level;
     uint32_t* totals = c->level_tile_ctr;
     c->launches += 4;
-    k_nodes_count<<<ntiles, kPBThreads, 0, c->stream>>>(c->tkey, n, leaf_cap, span, tile, ntiles);
+    (batch ? k_nodes_count<true> : k_nodes_count<false>)<<<ntiles, kPBThreads, 0, c->stream>>>(
+        c->tkey, c->body_sys, n, leaf_cap, span, tile, ntiles);
     k_nodes_scan<<<kMaxDepth, 1024, 0, c->stream>>>(tile, ntiles, totals);
-    k_nodes_write<<<ntiles, kPBThreads, 0, c->stream>>>(c->tkey, n, leaf_cap, span, tile, ntiles, totals, c->nkey,
-                                                        c->nrange, c->wnode, c->nchildbyte, c->nparent,
-                                                        c->level_bounds, (long long)c->node_cap, c->err);
+    (batch ? k_nodes_write<true> : k_nodes_write<false>)<<<ntiles, kPBThreads, 0, c->stream>>>(
+        c->tkey, c->body_sys, c->sys_off, batch ? c->nsys : 1, n, span, tile, ntiles, totals, c->nkey, c->nrange,
+        c->wnode, c->nchildbyte, c->nparent, c->level_bounds, (long long)c->node_cap, c->err);
     const int lgrid = (int)std::min<size_t>((size_t)c->sms * 8, (c->node_cap + kThreads - 1) / kThreads);
     k_nodes_link<<<lgrid, kThreads, 0, c->stream>>>(c->level_bounds, c->nkey, c->nparent, c->nrange, c->wnode,
                                                     c->nchildbyte, c->err);
