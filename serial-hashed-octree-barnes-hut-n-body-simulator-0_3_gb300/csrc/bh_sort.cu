@@ -259,22 +259,24 @@ __global__ __launch_bounds__(kThreads, BH_SORT_MIN_BLOCKS) void k_onesweep(const
 // ---------------------------------------------------------------------------------------
 // Small sorts: tiles and their merge (bh_tilesort.cuh), two launches
 // ---------------------------------------------------------------------------------------
-__global__ __launch_bounds__(kTileKeys) void k_tile_pairs(const uint64_t* __restrict__ kin,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(kTile) void k_tile_pairs(const uint64_t* __restrict__ kin,
                                                           const uint32_t* __restrict__ vin,
                                                           uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                           int n) {
-  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
-  tile_sort_store<false>(i < n ? kin[i] : ~0ull, i < n ? vin[i] : 0u, 0u, base, n, kout, vout);
+  const int base = blockIdx.x * kTile, i = base + threadIdx.x;
+  tile_sort_store<kTile, kSeg>(i < n ? kin[i] : ~0ull, i < n ? vin[i] : 0u, 0u, base, n, kout, vout);
 }
 
-__global__ __launch_bounds__(kMergeThreads) void k_merge_pairs(const uint64_t* __restrict__ kin,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(32 * kMergeParts) void k_merge_pairs(const uint64_t* __restrict__ kin,
                                                                const uint32_t* __restrict__ vin,
                                                                uint64_t* __restrict__ kout,
                                                                uint32_t* __restrict__ vout, int n) {
   int place;
   uint64_t key;
   uint32_t val;
-  if (!tile_merge_rank<false>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
+  if (!tile_merge_rank<kTile, kSeg>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
   kout[place] = key;
   vout[place] = val;
 }
@@ -304,8 +306,8 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
   if (n <= tile_sort_max() && first_pass == 0 && npasses == kPasses) {
     // the result goes back to keys_in / vals_in, as after the eight digit passes
     c->launches += 2;
-    k_tile_pairs<<<tile_blocks(n), kTileKeys, 0, st>>>(keys_in, vals_in, keys_tmp, vals_tmp, n);
-    k_merge_pairs<<<merge_blocks(n), kMergeThreads, 0, st>>>(keys_tmp, vals_tmp, keys_in, vals_in, n);
+    BH_TILE_KERNEL(k_tile_pairs, n, false)<<<tile_blocks(n), tile_keys(n), 0, st>>>(keys_in, vals_in, keys_tmp, vals_tmp, n);
+    BH_TILE_KERNEL(k_merge_pairs, n, false)<<<merge_blocks(n), merge_threads(n), 0, st>>>(keys_tmp, vals_tmp, keys_in, vals_in, n);
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);
@@ -406,7 +408,7 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
   }
   uint64_t* tmp_keys = (uint64_t*)(base + kOffTmpKeys);
   uint32_t* tmp_vals = (uint32_t*)(base + kOffTmpVals);
-  k_tile_pairs<<<tile_blocks(nn), kTileKeys, 0, st>>>(keys_in, vals_in, tmp_keys, tmp_vals, nn);
-  k_merge_pairs<<<merge_blocks(nn), kMergeThreads, 0, st>>>(tmp_keys, tmp_vals, keys_out, vals_out, nn);
+  BH_TILE_KERNEL(k_tile_pairs, nn, false)<<<tile_blocks(nn), tile_keys(nn), 0, st>>>(keys_in, vals_in, tmp_keys, tmp_vals, nn);
+  BH_TILE_KERNEL(k_merge_pairs, nn, false)<<<merge_blocks(nn), merge_threads(nn), 0, st>>>(tmp_keys, tmp_vals, keys_out, vals_out, nn);
   return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ERR_DEVICE;
 }

@@ -456,21 +456,21 @@ __global__ __launch_bounds__(kThreads) void k_gather_kd_treekey(
 // ---- systems small enough for the two-launch sort (tile_sort_max): the stages around it in its kernels
 
 // Morton keys, tile-sorted with their slots (kSeg: by the slots' systems first).
-template <bool kSeg>
-__global__ __launch_bounds__(kTileKeys) void k_morton_tiles(const float4* __restrict__ pos, int n,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(kTile) void k_morton_tiles(const float4* __restrict__ pos, int n,
                                                             const Geom* __restrict__ g,
                                                             const uint16_t* __restrict__ body_sys,
                                                             uint64_t* __restrict__ kout, uint32_t* __restrict__ vout) {
-  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  const int base = blockIdx.x * kTile, i = base + threadIdx.x;
   const uint32_t sys = kSeg ? (i < n ? (uint32_t)body_sys[i] : 0xffffffffu) : 0u;
   const uint64_t key = i < n ? morton_key(pos[i], kSeg ? g[sys] : *g) : ~0ull;
-  tile_sort_store<kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
+  tile_sort_store<kTile, kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
 }
 
 // The Morton merge, with k_gather_kd_treekey's work at each body's place in the sorted order: kout
 // (optional) receives the sorted keys, ktree the tree keys by slot.
-template <bool kSeg>
-__global__ __launch_bounds__(kMergeThreads) void k_merge_kd(
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(32 * kMergeParts) void k_merge_kd(
     const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, int n, const float4* __restrict__ pin,
     const float4* __restrict__ velin, const float4* __restrict__ acc, int acc_follows_body, float dt, float half_dt,
     const Geom* __restrict__ g, const uint16_t* __restrict__ body_sys, const uint32_t* __restrict__ off,
@@ -478,7 +478,7 @@ __global__ __launch_bounds__(kMergeThreads) void k_merge_kd(
   int j;
   uint64_t key;
   uint32_t i;
-  if (!tile_merge_rank<kSeg>(kin, vin, body_sys, off, n, j, key, i)) return;
+  if (!tile_merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, j, key, i)) return;
   float4 p = pin[i], v = velin[i];
   kick_drift(p, v, acc[acc_follows_body ? i : (uint32_t)j], dt, half_dt);
   pout[j] = p;
@@ -488,27 +488,28 @@ __global__ __launch_bounds__(kMergeThreads) void k_merge_kd(
 }
 
 // Tree keys (given, or of the positions), tile-sorted with their slots.
-template <bool kSeg>
-__global__ __launch_bounds__(kTileKeys) void k_tree_tiles(const uint64_t* __restrict__ ktree,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(kTile) void k_tree_tiles(const uint64_t* __restrict__ ktree,
                                                           const float4* __restrict__ pos, int n,
                                                           const Geom* __restrict__ g,
                                                           const uint16_t* __restrict__ body_sys,
                                                           uint64_t* __restrict__ kout, uint32_t* __restrict__ vout) {
-  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  const int base = blockIdx.x * kTile, i = base + threadIdx.x;
   const uint32_t sys = kSeg ? (i < n ? (uint32_t)body_sys[i] : 0xffffffffu) : 0u;
   const uint64_t key = i < n ? (ktree ? ktree[i] : tree_key(pos[i], *g)) : ~0ull;
-  tile_sort_store<kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
+  tile_sort_store<kTile, kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
 }
 
 // The half-kick and drift in place of order (the differentiable path), with the tree keys of the
 // drifted positions tile-sorted.
-__global__ __launch_bounds__(kTileKeys) void k_kd_tiles(const float4* __restrict__ pin,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(kTile) void k_kd_tiles(const float4* __restrict__ pin,
                                                         const float4* __restrict__ velin,
                                                         const float4* __restrict__ acc, int n, float dt, float half_dt,
                                                         const Geom* __restrict__ g, float4* __restrict__ pout,
                                                         float4* __restrict__ velout, uint64_t* __restrict__ kout,
                                                         uint32_t* __restrict__ vout) {
-  const int base = blockIdx.x * kTileKeys, i = base + threadIdx.x;
+  const int base = blockIdx.x * kTile, i = base + threadIdx.x;
   uint64_t key = ~0ull;
   if (i < n) {
     float4 p = pin[i], v = velin[i];
@@ -517,12 +518,12 @@ __global__ __launch_bounds__(kTileKeys) void k_kd_tiles(const float4* __restrict
     velout[i] = v;
     key = tree_key(p, *g);
   }
-  tile_sort_store<false>(key, (uint32_t)i, 0u, base, n, kout, vout);
+  tile_sort_store<kTile, kSeg>(key, (uint32_t)i, 0u, base, n, kout, vout);
 }
 
 // The tree-key merge, with the positions gathered into tree order.
-template <bool kSeg>
-__global__ __launch_bounds__(kMergeThreads) void k_merge_tree(const uint64_t* __restrict__ kin,
+template <int kTile, bool kSeg>
+__global__ __launch_bounds__(32 * kMergeParts) void k_merge_tree(const uint64_t* __restrict__ kin,
                                                               const uint32_t* __restrict__ vin, int n,
                                                               const float4* __restrict__ pos,
                                                               const uint16_t* __restrict__ body_sys,
@@ -533,7 +534,7 @@ __global__ __launch_bounds__(kMergeThreads) void k_merge_tree(const uint64_t* __
   int r;
   uint64_t key;
   uint32_t slot;
-  if (!tile_merge_rank<kSeg>(kin, vin, body_sys, off, n, r, key, slot)) return;
+  if (!tile_merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, r, key, slot)) return;
   tkey[r] = key;
   tslot[r] = slot;
   tpos[r] = pos[slot];
@@ -1155,16 +1156,16 @@ __device__ __forceinline__ void quad_add(float q[6], float m, float x, float y, 
 // supers, which bounds the work at 2^22 bodies, where the visits of a body per level would not.
 //   count <= 16     one thread in systems of more than 65 536 bodies (32 nodes per warp: the
 //                   fewest instructions); below that a team, whose chain of sums is shorter
-//   count <= 1024   a team of 8 lanes (128 without chunk records)
-//   count <= 16384  a warp (1024 without)
+//   count <= 1024   a team of 8 lanes (64 without chunk records)
+//   count <= 16384  a warp (256 without)
 //   larger          the block
 // The block collects the larger nodes of its tile and takes them after the small ones. Nodes are
 // numbered level by level, so the largest come first: the head of the list is dealt node by node to
 // all blocks, the rest in tiles of neighbouring nodes from a queue.
 constexpr int kThreadNode = 16;  // largest node of a thread
 constexpr int kTeam = 8;
-constexpr int kTeamDirect = 128, kTeamNode = 1024;  // largest node of a team without / with chunks
-constexpr int kWarpDirect = 1024, kWarpNode = 16384;
+constexpr int kTeamDirect = 64, kTeamNode = 1024;  // largest node of a team without / with chunks
+constexpr int kWarpDirect = 256, kWarpNode = 16384;
 constexpr int kChunk = 64;    // bodies per chunk record
 constexpr int kSuper = 64;    // chunks per super record
 
@@ -1814,14 +1815,14 @@ void launch_gather_kd_treekey(bh_ctx* c, const uint32_t* perm, int n, const floa
 // pairs pass through keys[1] / vals[1].
 void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  (batch ? k_morton_tiles<true> : k_morton_tiles<false>)<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(
+  BH_TILE_KERNEL(k_morton_tiles, n, batch)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
       pos, n, batch ? c->sys_geom : c->geom, c->body_sys, c->keys[1], c->vals[1]);
 }
 
 void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
                      float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch) {
   c->launches += 1;
-  (batch ? k_merge_kd<true> : k_merge_kd<false>)<<<merge_blocks(n), kMergeThreads, 0, c->stream>>>(
+  BH_TILE_KERNEL(k_merge_kd, n, batch)<<<merge_blocks(n), merge_threads(n), 0, c->stream>>>(
       c->keys[1], c->vals[1], n, pin, vin, acc, acc_follows_body, dt, 0.5f * dt, batch ? c->sys_geom : c->geom,
       c->body_sys, c->sys_off, pout, vout, kout, ktree);
 }
@@ -1829,19 +1830,19 @@ void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, con
 void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
                      float4* vout) {
   c->launches += 1;
-  k_kd_tiles<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(pin, vin, acc, n, dt, 0.5f * dt, c->geom, pout, vout,
+  BH_TILE_KERNEL(k_kd_tiles, n, false)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(pin, vin, acc, n, dt, 0.5f * dt, c->geom, pout, vout,
                                                           c->keys[1], c->vals[1]);
 }
 
 void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  (batch ? k_tree_tiles<true> : k_tree_tiles<false>)<<<tile_blocks(n), kTileKeys, 0, c->stream>>>(
+  BH_TILE_KERNEL(k_tree_tiles, n, batch)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
       ktree, pos, n, c->geom, c->body_sys, c->keys[1], c->vals[1]);
 }
 
 void launch_merge_tree(bh_ctx* c, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  (batch ? k_merge_tree<true> : k_merge_tree<false>)<<<merge_blocks(n), kMergeThreads, 0, c->stream>>>(
+  BH_TILE_KERNEL(k_merge_tree, n, batch)<<<merge_blocks(n), merge_threads(n), 0, c->stream>>>(
       c->keys[1], c->vals[1], n, pos, c->body_sys, c->sys_off, c->tkey, c->tslot, c->tpos);
 }
 
