@@ -101,11 +101,13 @@ struct Counters {
 
 // The small device results of a context in one block: cleared up to `level_bounds` with one memset at
 // the start of a step and read back whole with one copy at its end.
+constexpr int kDiagSums = 12;  // sums of the conservation diagnostics
 struct Status {
   Counters counters;
   uint32_t err;
   int level_bounds[kLevels + 2];
   Geom geom;
+  double sums[kDiagSums];
 };
 
 // Radix sort (onesweep) scratch.
@@ -307,6 +309,8 @@ void launch_lookup(bh_ctx* c, uint64_t key, int* out_index);
 void launch_walk_record(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick, float half_dt,
                         Chunk* tape, unsigned* tape_count, int tape_cap);
 void launch_fp32_peak(cudaStream_t st, float* sink, int blocks);
+// The potential of every body over the current tree, by slot (clear_device_flags before it).
+void launch_potential(bh_ctx* c, int n, float theta, float eps, int mode, float* pot_slot);
 // Launch shapes of the quadrupole walk (positive softening) that bh_autotune_walk times.
 struct WalkVariant {
   int warps, min_blocks, stack, form, regs, group;  // group: bodies per warp (single systems)

@@ -230,6 +230,67 @@ __device__ __forceinline__ void eval_points(Smem& s, int cnt, const WalkNode* __
   acc.add(bx, by, bz);
 }
 
+// The potential's terms (diagnostics): M / D + d.Q.d / (2 D^5) of a cell, m / D of a point at another
+// position than the body's. phi = -sum, every term added to a compensated per-lane sum (acc.sx).
+template <bool kCells, int kGroup, class Smem>
+__device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode* __restrict__ nodes,
+                                               const float4* __restrict__ tpos, int lane, float px, float py, float pz,
+                                               float eps2, Acc& acc) {
+  constexpr int kSlots = 32 / kGroup;
+  const int slot = lane / kGroup;
+  const uint32_t lanebit = 1u << (lane % kGroup);
+  __syncwarp();
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v, v2 = v;  // lanes past cnt: empty mask
+  if (lane < cnt) {
+    if (kCells) {
+      const WalkNode* nd = nodes + s.cell_node[lane];
+      v = __ldg(&nd->mac);
+      v1 = __ldg(&nd->mq);
+      v2 = __ldg(&nd->q2);
+      v2.w = __uint_as_float(s.cell_mask[lane]);
+    } else {
+      const int e = s.pt_idx[lane];
+      v2.w = __uint_as_float(s.pt_mask[lane]);
+      if (e >= 0) {
+        v = __ldg(tpos + e);
+      } else {
+        const WalkNode* nd = nodes + (-e - 1);
+        const float4 mac = __ldg(&nd->mac);
+        v = make_float4(mac.x, mac.y, mac.z, __ldg(&nd->mq.x));
+      }
+    }
+  }
+  s.st0[lane] = v;
+  if (kCells) s.st1[lane] = v1;
+  s.st2[lane] = v2;
+  __syncwarp();
+#pragma unroll 4
+  for (int r = 0; r < cnt; r += kSlots) {
+    const int j = r + slot;
+    const float4 c0 = s.st0[j], c2 = s.st2[j];
+    const float dx = c0.x - px, dy = c0.y - py, dz = c0.z - pz;
+    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float rinv = rsqrtf(d2 + eps2);
+    bool take = (__float_as_uint(c2.w) & lanebit) != 0u;
+    float term;
+    if (kCells) {
+      const float4 c1 = s.st1[j];
+      const float qx = fmaf(c1.y, dx, fmaf(c1.z, dy, c1.w * dz));
+      const float qy = fmaf(c1.z, dx, fmaf(c2.x, dy, c2.y * dz));
+      const float qz = fmaf(c1.w, dx, fmaf(c2.y, dy, c2.z * dz));
+      const float qr = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
+      const float u = rinv * rinv;
+      term = fmaf(0.5f * qr, rinv * u * u, c1.x * rinv);
+    } else {
+      term = c0.w * rinv;
+      take = take && !((dx == 0.f) & (dy == 0.f) & (dz == 0.f));
+    }
+    const float y = (take ? -term : 0.f) - acc.cx, t = acc.sx + y;
+    acc.cx = (t - acc.sx) - y;
+    acc.sx = t;
+  }
+}
+
 // Moves buffer entries [32, n) to [0, n - 32) after the first 32 were evaluated.
 __device__ __forceinline__ void shift_down(int* idx, uint32_t* msk, int n, int lane) {
   __syncwarp();
@@ -247,7 +308,7 @@ __device__ __forceinline__ void shift_down(int* idx, uint32_t* msk, int n, int l
   }
 }
 
-template <bool kQuad, bool kSelfTest, bool kRec = false, class Cfg = CfgDefault, int kGroup = 32>
+template <bool kQuad, bool kSelfTest, bool kRec = false, class Cfg = CfgDefault, int kGroup = 32, bool kPot = false>
 __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const WalkNode* __restrict__ nodes,
                                                    const float4* __restrict__ tpos,
                                                    const uint32_t* __restrict__ tslot, int n, float theta2,
@@ -321,6 +382,18 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
       bmaxz = fmaxf(bmaxz, __shfl_xor_sync(0xffffffffu, bmaxz, o));
     }
     Acc acc;
+    auto run_cells = [&](int cnt) {
+      if (kPot)
+        eval_potential<true, kGroup>(s, cnt, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc);
+      else
+        eval_cells<kRec, Cfg::kForm, kGroup>(s, cnt, nodes, lane, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
+    };
+    auto run_points = [&](int cnt) {
+      if (kPot)
+        eval_potential<false, kGroup>(s, cnt, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc);
+      else
+        eval_points<kSelfTest, kRec, kGroup>(s, cnt, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+    };
     int sp = 0, ncell = 0, npt = 0;
     // per-lane shares of the group's interaction counts (each lane counts the entries it
     // appended, times the lanes in their masks); self pairs are subtracted
@@ -336,7 +409,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           s.pt_mask[lane] = active;
         }
         if (lane == 0) cnt_pt += (long long)k * __popc(active);
-        eval_points<kSelfTest, kRec, kGroup>(s, k, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+        run_points(k);
       }
       if (lane == 0) cnt_pt -= __popc(active);
     } else {
@@ -473,7 +546,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           }
           ncell += __popc(bal);
           if (ncell >= 32) {
-            eval_cells<kRec, Cfg::kForm, kGroup>(s, 32, nodes, lane, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
+            run_cells(32);
             shift_down(s.cell_node, s.cell_mask, ncell, lane);
             ncell -= 32;
           }
@@ -491,7 +564,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           }
           npt += __popc(bal);
           if (npt >= 32) {
-            eval_points<kSelfTest, kRec, kGroup>(s, 32, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+            run_points(32);
             shift_down(s.pt_idx, s.pt_mask, npt, lane);
             npt -= 32;
           }
@@ -550,7 +623,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
           }
           npt += kk;
           if (npt >= 32) {
-            eval_points<kSelfTest, kRec, kGroup>(s, 32, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+            run_points(32);
             shift_down(s.pt_idx, s.pt_mask, npt, lane);
             npt -= 32;
           }
@@ -598,7 +671,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
             }
             npt += kk;
             if (npt >= 32) {
-              eval_points<kSelfTest, kRec, kGroup>(s, 32, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+              run_points(32);
               shift_down(s.pt_idx, s.pt_mask, npt, lane);
               npt -= 32;
             }
@@ -607,8 +680,8 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         }
       }
     }
-    if (ncell > 0) eval_cells<kRec, Cfg::kForm, kGroup>(s, ncell, nodes, lane, p.x, p.y, p.z, eps2, acc, ev_cell, rec);
-    if (npt > 0) eval_points<kSelfTest, kRec, kGroup>(s, npt, nodes, tpos, lane, p.x, p.y, p.z, eps2, acc, ev_pt, rec);
+    if (ncell > 0) run_cells(ncell);
+    if (npt > 0) run_points(npt);
     if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
 #pragma unroll
       for (int o = kGroup; o < 32; o <<= 1) {
@@ -622,7 +695,9 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         acc.add(ox, oy, oz);
       }
     }
-    if (valid && slot == 0) {
+    if (kPot) {  // acc_slot receives one float per body
+      if (valid && slot == 0) reinterpret_cast<float*>(acc_slot)[__ldg(tslot + i)] = acc.sx;
+    } else if (valid && slot == 0) {
       const uint32_t bslot = __ldg(tslot + i);
       const float ax = acc.sx, ay = acc.sy, az = acc.sz;
       acc_slot[bslot] = make_float4(ax, ay, az, 0.f);
@@ -662,7 +737,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
 // Persistent grid of one walk instantiation on the current device: every block that can be
 // resident at once (kept per device; bh_create fills it through walk_init before any capture).
 constexpr int kWalkMaxDevices = 64;
-template <bool kQuad, bool kSelf, bool kRec, class Cfg, int kGroup = 32>
+template <bool kQuad, bool kSelf, bool kRec, class Cfg, int kGroup = 32, bool kPot = false>
 int walk_grid() {
   static int blocks[kWalkMaxDevices] = {};
   int dev = 0;
@@ -673,7 +748,7 @@ int walk_grid() {
   if (blocks[dev] == 0) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk<kQuad, kSelf, kRec, Cfg, kGroup>, Cfg::kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk<kQuad, kSelf, kRec, Cfg, kGroup, kPot>, Cfg::kThreads, 0);
     blocks[dev] = max(1, sms * max(1, per_sm));
   }
   return blocks[dev];
@@ -772,6 +847,37 @@ void launch_quad_variant(bh_ctx* c, int v, int n, const WalkArgs& a) {
 }  // namespace
 
 int walk_variants() { return kVariants; }
+
+// The potential of every body (kPot), phi by slot: the diagnostics' walk, with the force walk's groups.
+namespace {
+template <bool kQuad, int kGroup>
+void launch_potential_t(bh_ctx* c, int n, float theta2, float eps2, float* pot_slot) {
+  const int ngroups = (n + kGroup - 1) / kGroup;
+  const int grid = min(walk_grid<kQuad, true, false, CfgDefault, kGroup, true>(), ngroups);
+  k_walk<kQuad, true, false, CfgDefault, kGroup, true><<<grid, CfgDefault::kThreads, 0, c->stream>>>(
+      c->wnode, c->tpos, c->tslot, n, theta2, eps2, reinterpret_cast<float4*>(pot_slot), nullptr, 0.f, nullptr, nullptr,
+      0, c->counters, c->err);
+}
+
+template <bool kQuad>
+void launch_potential_group(bh_ctx* c, int n, float theta2, float eps2, float* pot_slot) {
+  switch (walk_group_size(n)) {
+    case 4: launch_potential_t<kQuad, 4>(c, n, theta2, eps2, pot_slot); break;
+    case 8: launch_potential_t<kQuad, 8>(c, n, theta2, eps2, pot_slot); break;
+    case 16: launch_potential_t<kQuad, 16>(c, n, theta2, eps2, pot_slot); break;
+    default: launch_potential_t<kQuad, 32>(c, n, theta2, eps2, pot_slot); break;
+  }
+}
+}  // namespace
+
+void launch_potential(bh_ctx* c, int n, float theta, float eps, int mode, float* pot_slot) {
+  if (n <= 0) return;
+  c->launches += 1;
+  if (mode == BH_MULTIPOLE_QUADRUPOLE)
+    launch_potential_group<true>(c, n, theta * theta, eps * eps, pot_slot);
+  else
+    launch_potential_group<false>(c, n, theta * theta, eps * eps, pot_slot);
+}
 
 // Small groups give more warps and, with their boxes, fewer entries a body (at 16 384 bodies, leaf
 // capacity 1, a group of 32 / 16 / 8 evaluates 2200 / 1835 / 1569 entries), but each group traverses

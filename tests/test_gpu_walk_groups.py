@@ -57,3 +57,32 @@ def test_small_ensemble_groups_match_single_systems(bh):
             sl = slice(off[s], off[s + 1])
             assert np.allclose(bp[sl], p, rtol=0, atol=1e-6) and np.allclose(bv[sl], v, rtol=0, atol=1e-6)
             assert float(np.percentile(relerr(ba[sl], a), 99)) <= 1e-5
+
+
+@pytest.mark.parametrize("n,leaf,mode", [(2, 1, 1), (33, 4, 0), (1001, 1, 1), (12289, 8, 1), (24577, 8, 0), (196609, 16, 1)])
+def test_potential_of_every_group_size(bh, n, leaf, mode):
+    """phi at theta = 0 is the direct sum (coincident bodies left out); at theta = 0.5 it follows it within the
+    quadrupole tree's accuracy. FP64 reference on a seeded subset of the bodies."""
+    pm, vel = bh.plummer(60 + n, n)
+    if n > 100:
+        pm[7, :3] = pm[70, :3]
+    eps = 0.01
+    rng = np.random.default_rng(n)
+    with bh.Simulation(n) as sim:
+        sim.set_bodies(pm, vel)
+        c, size = sim.bounds()
+        sim.build(c, 2 * size, leaf, mode)
+        e0, phi0 = sim.energy(0.0, eps, potential=True) if n < 50000 else (None, None)
+        e1, phi1 = sim.energy(0.5, eps, potential=True)
+    x, m = pm[:, :3].astype(np.float64), pm[:, 3].astype(np.float64)
+    pick = np.unique(np.concatenate([rng.integers(0, n, 60), [0, min(7, n - 1), min(70, n - 1)]]))
+    ref = np.empty(len(pick))
+    for k, i in enumerate(pick):
+        r2 = ((x - x[i]) ** 2).sum(1)
+        ref[k] = -(m[r2 > 0] / np.sqrt(r2[r2 > 0] + eps * eps)).sum()
+    if phi0 is not None:
+        # n terms in FP32 with a compensated sum: rsqrt (2 ulp) and the rounding of each term
+        assert np.all(np.abs(phi0[pick] - ref) <= 1e-6 * np.abs(ref) + 1e-12)
+        assert abs(e0["potential"] - 0.5 * float((m * phi0).sum())) <= 1e-9 * abs(e0["potential"])
+    if mode:
+        assert np.median(np.abs(phi1[pick] - ref) / np.abs(ref).clip(1e-12)) <= 1e-3
