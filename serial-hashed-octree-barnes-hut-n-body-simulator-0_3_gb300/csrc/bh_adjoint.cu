@@ -105,28 +105,40 @@ struct VjpWarp {
   float g[3][kVjpHalf][33];
 };
 
-// Lane b of the half [h, h + 16) sums its body's row over the chunk's entries; d = source -
-// body, so the body's own position takes the negative.
+// One reduction of four floats to L2 (16-byte aligned).
+__device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w)
+               : "memory");
+}
+
+// The rows of the half [h, h + 16) summed over the chunk's entries, two lanes per body (16 entries
+// each); d = source - body, so the body's own position takes the negative.
 __device__ __forceinline__ void vjp_rows(VjpWarp& s, int h, int hend, int lane, int cnt, uint32_t my_slot,
                                          float4* __restrict__ xbar) {
   __syncwarp();
-  if (lane >= h && lane < hend) {
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    for (int k = 0; k < cnt; ++k) {
-      sx += s.g[0][lane - h][k];
-      sy += s.g[1][lane - h][k];
-      sz += s.g[2][lane - h][k];
+  const int b = lane % kVjpHalf, k0 = lane / kVjpHalf * 16, k1 = min(cnt, k0 + 16);
+  float sx = 0.f, sy = 0.f, sz = 0.f;
+  if (h + b < hend)
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      sx += s.g[0][b][k];
+      sy += s.g[1][b][k];
+      sz += s.g[2][b][k];
     }
-    atomicAdd(&xbar[my_slot].x, -sx);
-    atomicAdd(&xbar[my_slot].y, -sy);
-    atomicAdd(&xbar[my_slot].z, -sz);
-  }
+  sx += __shfl_xor_sync(0xffffffffu, sx, kVjpHalf);
+  sy += __shfl_xor_sync(0xffffffffu, sy, kVjpHalf);
+  sz += __shfl_xor_sync(0xffffffffu, sz, kVjpHalf);
+  // lane h + b holds the slot of body h + b
+  if (lane >= h && lane < hend) red_add4(&xbar[my_slot].x, -sx, -sy, -sz, 0.f);
   __syncwarp();
 }
 
 constexpr int kVjpWarps = 4;
 constexpr size_t kVjpSmem = sizeof(VjpWarp) * kVjpWarps;
 
+// Bound by issue (about 90 instructions per entry and body, lanes outside the mask idle) with the node
+// adjoints' reductions to L2 beside it; at 65 536 bodies 770 us a step with scalar atomics, half the
+// lanes summing the rows and the node's Qb terms formed one by one, 550 so.
 // Replays the recorded chunks, one warp per chunk, lane = buffer entry: each lane loops over the
 // group's bodies, sums its entry's adjoints (node or source body) in registers and leaves the
 // body-side term in the table; then lane b sums row b for body b.
@@ -197,29 +209,23 @@ __global__ __launch_bounds__(kVjpWarps * 32) void k_vjp(const Chunk* __restrict_
         cby += gy;
         cbz += gz;
         mb = fmaf(w3, ad, mb);
-        const float h25 = 2.5f * w7 * ad;
-        const float ax = take ? ab.x : 0.f, ay = take ? ab.y : 0.f, az = take ? ab.z : 0.f;
-        bxx += fmaf(-w5 * ax, dx, h25 * dx * dx);
-        byy += fmaf(-w5 * ay, dy, h25 * dy * dy);
-        bzz += fmaf(-w5 * az, dz, h25 * dz * dz);
-        bxy += fmaf(-w5, fmaf(ax, dy, ay * dx), 2.f * h25 * dx * dy);
-        bxz += fmaf(-w5, fmaf(ax, dz, az * dx), 2.f * h25 * dx * dz);
-        byz += fmaf(-w5, fmaf(ay, dz, az * dy), 2.f * h25 * dy * dz);
+        // Qb += e d^T + d e^T on and off the diagonal, e = h25 d - w5 ab (zero outside the mask)
+        const float h25 = 0.5f * cq;
+        const float ex = fmaf(h25, dx, -w5t * ab.x), ey = fmaf(h25, dy, -w5t * ab.y), ez = fmaf(h25, dz, -w5t * ab.z);
+        bxx = fmaf(ex, dx, bxx);
+        byy = fmaf(ey, dy, byy);
+        bzz = fmaf(ez, dz, bzz);
+        bxy = fmaf(ex, dy, fmaf(ey, dx, bxy));
+        bxz = fmaf(ex, dz, fmaf(ez, dx, bxz));
+        byz = fmaf(ey, dz, fmaf(ez, dy, byz));
       }
       vjp_rows(s, h, hend, lane, cnt, my_slot, xbar);
       }
       if (has && mk) {
         float* a = nadj + (size_t)e * kNadj;
-        atomicAdd(a + 0, cbx);
-        atomicAdd(a + 1, cby);
-        atomicAdd(a + 2, cbz);
-        atomicAdd(a + 3, mb);
-        atomicAdd(a + 4, bxx);
-        atomicAdd(a + 5, bxy);
-        atomicAdd(a + 6, bxz);
-        atomicAdd(a + 7, byy);
-        atomicAdd(a + 8, byz);
-        atomicAdd(a + 9, bzz);
+        red_add4(a, cbx, cby, cbz, mb);
+        red_add4(a + 4, bxx, bxy, bxz, byy);
+        red_add4(a + 8, byz, bzz, 0.f, 0.f);
       }
     } else {
       const int src = has ? (e >= 0 ? e : nodes[-e - 1].link.z) : 0;  // a point node is a single-body leaf
@@ -252,9 +258,7 @@ __global__ __launch_bounds__(kVjpWarps * 32) void k_vjp(const Chunk* __restrict_
       }
       if (has && mk) {
         const uint32_t ss = tslot[src];
-        atomicAdd(&xbar[ss].x, tx);
-        atomicAdd(&xbar[ss].y, ty);
-        atomicAdd(&xbar[ss].z, tz);
+        red_add4(&xbar[ss].x, tx, ty, tz, 0.f);
         atomicAdd(&mbar[ss], tm);
       }
     }

@@ -284,6 +284,7 @@ int tile_sort_max();
 void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch = false);
 void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
                      float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch = false);
+// (in the order of c->tslot, a permutation of the n bodies: the previous tree's)
 void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
                      float4* vout);
 void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch = false);

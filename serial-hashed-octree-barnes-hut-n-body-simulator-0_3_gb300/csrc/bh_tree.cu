@@ -500,25 +500,30 @@ __global__ __launch_bounds__(kTile) void k_tree_tiles(const uint64_t* __restrict
   tile_sort_store<kTile, kSeg>(key, (uint32_t)i, sys, base, n, kout, vout);
 }
 
-// The half-kick and drift in place of order (the differentiable path), with the tree keys of the
-// drifted positions tile-sorted.
+// The half-kick and drift of bodies that keep their slots (the differentiable path), with the tree keys
+// of the drifted positions tile-sorted. The bodies are taken in the previous tree order, in which
+// the new keys are nearly sorted and the merge has little to search (65 536 bodies: 75 -> 35 us
+// against slot order); bodies of one key keep that order.
 template <int kTile, bool kSeg>
 __global__ __launch_bounds__(kTile) void k_kd_tiles(const float4* __restrict__ pin,
                                                         const float4* __restrict__ velin,
-                                                        const float4* __restrict__ acc, int n, float dt, float half_dt,
-                                                        const Geom* __restrict__ g, float4* __restrict__ pout,
-                                                        float4* __restrict__ velout, uint64_t* __restrict__ kout,
-                                                        uint32_t* __restrict__ vout) {
-  const int base = blockIdx.x * kTile, i = base + threadIdx.x;
+                                                        const float4* __restrict__ acc,
+                                                        const uint32_t* __restrict__ order, int n, float dt,
+                                                        float half_dt, const Geom* __restrict__ g,
+                                                        float4* __restrict__ pout, float4* __restrict__ velout,
+                                                        uint64_t* __restrict__ kout, uint32_t* __restrict__ vout) {
+  const int base = blockIdx.x * kTile, k = base + threadIdx.x;
   uint64_t key = ~0ull;
-  if (i < n) {
+  uint32_t i = 0;
+  if (k < n) {
+    i = min(order[k], (uint32_t)n - 1u);
     float4 p = pin[i], v = velin[i];
     kick_drift(p, v, acc[i], dt, half_dt);
     pout[i] = p;
     velout[i] = v;
     key = tree_key(p, *g);
   }
-  tile_sort_store<kTile, kSeg>(key, (uint32_t)i, 0u, base, n, kout, vout);
+  tile_sort_store<kTile, kSeg>(key, i, 0u, base, n, kout, vout);
 }
 
 // The tree-key merge, with the positions gathered into tree order.
@@ -1830,8 +1835,8 @@ void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, con
 void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
                      float4* vout) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_kd_tiles, n, false)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(pin, vin, acc, n, dt, 0.5f * dt, c->geom, pout, vout,
-                                                          c->keys[1], c->vals[1]);
+  BH_TILE_KERNEL(k_kd_tiles, n, false)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
+      pin, vin, acc, c->tslot, n, dt, 0.5f * dt, c->geom, pout, vout, c->keys[1], c->vals[1]);
 }
 
 void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch) {
