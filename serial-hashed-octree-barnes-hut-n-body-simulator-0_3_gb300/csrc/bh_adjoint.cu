@@ -562,7 +562,7 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
   }
   BH_TRY(ensure_nodes(c, std::max<size_t>(2 * c->n + 64, 1024)));
   // a(x_0), recorded once to size the tape
-  if (a->chunk_cap == 0) a->chunk_cap = (c->n / 32 + 1) * 64;
+  if (a->chunk_cap == 0) a->chunk_cap = (c->n / record_group_size(c->n) + 1) * 64;
   if (a->tape.size() < 1) a->tape.resize(1);
   cudaEvent_t e0 = c->stage_ev[0], e1 = c->stage_ev[1];
   const uint64_t launches0 = c->launches;

@@ -320,6 +320,8 @@ int walk_variants();
 WalkVariant walk_variant_info(int v, size_t n);
 // Bodies per walk group for n bodies in all (a single system, or the systems of an ensemble).
 int walk_group_size(size_t n);
+// Bodies per group of the recording walk.
+int record_group_size(size_t n);
 void launch_walk_variant(bh_ctx* c, int v, int n, float theta, float eps, float4* acc_out, bool batch);
 
 // Frees the differentiable-path state of the context.
