@@ -141,6 +141,7 @@ __device__ __forceinline__ bool tile_merge_rank(const uint64_t* __restrict__ kin
         for (int q = 0; q < kFlight; ++q) {
           const int src = open ? __ffs(open) - 1 : 0;
           clo[q] = __shfl_sync(0xffffffffu, lo, src);
+          if (!open) clo[q] = 0;  // an empty search reads key 0
           clen[q] = open ? __shfl_sync(0xffffffffu, len, src) : 0;
           earlier[q] = t0 + src < own;
           open &= open - 1;
