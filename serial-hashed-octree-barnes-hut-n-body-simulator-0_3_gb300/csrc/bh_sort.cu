@@ -258,12 +258,19 @@ __global__ __launch_bounds__(kThreads, BH_SORT_MIN_BLOCKS) void k_onesweep(const
 
 // ---------------------------------------------------------------------------------------
 // Small sorts: tiles and their merge (bh_tilesort.cuh), two launches
+//
+// The merge is launched as a dependent of the tiles (programmatic stream serialization): its blocks are
+// set up while the tiles are sorted, and wait for them before they read. The gap between the two was a
+// tenth of the whole: bh_sort_keys_static, 40001 pairs, 56 us to 49.6 us. The kernels of a step don't do
+// this: between the nodes of its captured graph the gap is short already (1000 to 16384 bodies
+// unchanged, 48 small systems 7% slower).
 // ---------------------------------------------------------------------------------------
 template <int kTile, bool kSeg>
 __global__ __launch_bounds__(kTile) void k_tile_pairs(const uint64_t* __restrict__ kin,
                                                           const uint32_t* __restrict__ vin,
                                                           uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                           int n) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int base = blockIdx.x * kTile, i = base + threadIdx.x;
   tile_sort_store<kTile, kSeg>(i < n ? kin[i] : ~0ull, i < n ? vin[i] : 0u, 0u, base, n, kout, vout);
 }
@@ -273,12 +280,30 @@ __global__ __launch_bounds__(32 * kMergeParts) void k_merge_pairs(const uint64_t
                                                                const uint32_t* __restrict__ vin,
                                                                uint64_t* __restrict__ kout,
                                                                uint32_t* __restrict__ vout, int n) {
+  // the pointers pass through the wait, so no load through them can be moved before it
+  asm volatile("griddepcontrol.wait;" : "+l"(kin), "+l"(vin)::"memory");
   int place;
   uint64_t key;
   uint32_t val;
   if (!tile_merge_rank<kTile, kSeg>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
   kout[place] = key;
   vout[place] = val;
+}
+
+void launch_tile_sort(const uint64_t* kin, const uint32_t* vin, uint64_t* ktmp, uint32_t* vtmp, uint64_t* kout,
+                      uint32_t* vout, int n, cudaStream_t st) {
+  BH_TILE_KERNEL(k_tile_pairs, n, false)<<<tile_blocks(n), tile_keys(n), 0, st>>>(kin, vin, ktmp, vtmp, n);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(merge_blocks(n));
+  cfg.blockDim = dim3(merge_threads(n));
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, BH_TILE_KERNEL(k_merge_pairs, n, false), (const uint64_t*)ktmp, (const uint32_t*)vtmp,
+                     kout, vout, n);
 }
 
 }  // namespace
@@ -306,8 +331,7 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
   if (n <= tile_sort_max() && first_pass == 0 && npasses == kPasses) {
     // the result goes back to keys_in / vals_in, as after the eight digit passes
     c->launches += 2;
-    BH_TILE_KERNEL(k_tile_pairs, n, false)<<<tile_blocks(n), tile_keys(n), 0, st>>>(keys_in, vals_in, keys_tmp, vals_tmp, n);
-    BH_TILE_KERNEL(k_merge_pairs, n, false)<<<merge_blocks(n), merge_threads(n), 0, st>>>(keys_tmp, vals_tmp, keys_in, vals_in, n);
+    launch_tile_sort(keys_in, vals_in, keys_tmp, vals_tmp, keys_in, vals_in, n, st);
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);
@@ -408,7 +432,6 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
   }
   uint64_t* tmp_keys = (uint64_t*)(base + kOffTmpKeys);
   uint32_t* tmp_vals = (uint32_t*)(base + kOffTmpVals);
-  BH_TILE_KERNEL(k_tile_pairs, nn, false)<<<tile_blocks(nn), tile_keys(nn), 0, st>>>(keys_in, vals_in, tmp_keys, tmp_vals, nn);
-  BH_TILE_KERNEL(k_merge_pairs, nn, false)<<<merge_blocks(nn), merge_threads(nn), 0, st>>>(tmp_keys, tmp_vals, keys_out, vals_out, nn);
+  launch_tile_sort(keys_in, vals_in, tmp_keys, tmp_vals, keys_out, vals_out, nn, st);
   return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ERR_DEVICE;
 }
