@@ -963,9 +963,10 @@ bh_status bh_measure_fp32_peak(bh_ctx* c, double* tflops) {
 namespace {
 
 constexpr size_t kMaxSystems = 65535;  // system ids are stored as u16
-// Ensembles up to this size, of systems up to that one, sort in two launches by system and key, not in
-// ten passes over all bodies: key + tree sort (with the gathers) of 58 726 bodies in 48 systems up
+// Ensembles up to kBatchTileAny bodies, or up to kBatchTileMax of systems up to kBatchTileSystem, sort in
+// two launches by system and key, not in ten passes over all bodies: key + tree sort (with the gathers) of 58 726 bodies in 48 systems up
 // to 4 096 54 against 177 us, of 545 725 261 against 285, but of 4.2e6 1.97 against 1.14 ms.
+constexpr size_t kBatchTileAny = 98304;
 constexpr size_t kBatchTileMax = 393216;
 constexpr uint32_t kBatchTileSystem = 16384;
 
@@ -1116,7 +1117,7 @@ bh_status batch_layout(bh_ctx* c, const uint32_t* sys_offsets, size_t nsys) {
   BH_TRY(dalloc(&c->groups, groups.size()));
   c->ngroups = (int)groups.size();
   c->batch_group = (int)gsize;
-  c->batch_tiles = n <= (size_t)tile_sort_max() || (n <= kBatchTileMax && largest <= kBatchTileSystem);
+  c->batch_tiles = n <= kBatchTileAny || (n <= kBatchTileMax && largest <= kBatchTileSystem);
   cudaMemcpyAsync(c->sys_off, sys_offsets, sizeof(uint32_t) * (nsys + 1), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->body_sys, bs.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->groups, groups.data(), sizeof(int4) * groups.size(), cudaMemcpyHostToDevice, c->stream);

@@ -279,8 +279,9 @@ void launch_gather(bh_ctx* c, const uint32_t* perm, int n, const float4* pin, co
 void launch_gather_kd_treekey(bh_ctx* c, const uint32_t* perm, int n, const float4* pin, const float4* vin,
                               const float4* acc, int acc_follows_body, float dt, float4* pout, float4* vout,
                               uint64_t* tkeys, uint32_t* tidx, bool batch = false);
-// Single systems of at most this many bodies sort in two launches (bh_tilesort.cuh).
+// Single systems of at most this many bodies sort by tiles, in two or three launches (bh_tilesort.cuh).
 int tile_sort_max();
+void launch_merge_spans(bh_ctx* c, int n, uint64_t* kout, uint32_t* vout);
 void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch = false);
 void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
                      float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch = false);

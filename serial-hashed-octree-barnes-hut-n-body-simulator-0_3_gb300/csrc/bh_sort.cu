@@ -257,19 +257,17 @@ __global__ __launch_bounds__(kThreads, BH_SORT_MIN_BLOCKS) void k_onesweep(const
 }
 
 // ---------------------------------------------------------------------------------------
-// Small sorts: tiles and their merge (bh_tilesort.cuh), two launches
+// Small sorts: tiles and their merges (bh_tilesort.cuh), two or three launches
 //
-// The merge is launched as a dependent of the tiles (programmatic stream serialization): its blocks are
-// set up while the tiles are sorted, and wait for them before they read. The gap between the two was a
-// tenth of the whole: bh_sort_keys_static, 40001 pairs, 56 us to 49.6 us. The kernels of a step don't do
-// this: between the nodes of its captured graph the gap is short already (1000 to 16384 bodies
-// unchanged, 48 small systems 7% slower).
+// A merge is launched as a dependent of the kernel before it (programmatic stream serialization): its
+// blocks are set up while that one runs, and wait for it before they read. The gap between the two was
+// a tenth of the whole: bh_sort_keys_static, 40001 pairs in two launches, 56 us to 49.6 us. The kernels
+// of a step don't do this: between the nodes of its captured graph the gap is short already (1000 to
+// 16384 bodies unchanged, 48 small systems 7% slower).
 // ---------------------------------------------------------------------------------------
 template <int kTile, bool kSeg>
-__global__ __launch_bounds__(kTile) void k_tile_pairs(const uint64_t* __restrict__ kin,
-                                                          const uint32_t* __restrict__ vin,
-                                                          uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                          int n) {
+__global__ __launch_bounds__(kTile) void k_tile_pairs(const uint64_t* kin, const uint32_t* vin, uint64_t* kout,
+                                                      uint32_t* vout, int n) {  // in place or not
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int base = blockIdx.x * kTile, i = base + threadIdx.x;
   tile_sort_store<kTile, kSeg>(i < n ? kin[i] : ~0ull, i < n ? vin[i] : 0u, 0u, base, n, kout, vout);
@@ -285,33 +283,74 @@ __global__ __launch_bounds__(32 * kMergeParts) void k_merge_pairs(const uint64_t
   int place;
   uint64_t key;
   uint32_t val;
-  if (!tile_merge_rank<kTile, kSeg>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
+  if (!merge_rank<kTile, kSeg>(kin, vin, nullptr, nullptr, n, place, key, val)) return;
   kout[place] = key;
   vout[place] = val;
 }
 
-void launch_tile_sort(const uint64_t* kin, const uint32_t* vin, uint64_t* ktmp, uint32_t* vtmp, uint64_t* kout,
-                      uint32_t* vout, int n, cudaStream_t st) {
-  BH_TILE_KERNEL(k_tile_pairs, n, false)<<<tile_blocks(n), tile_keys(n), 0, st>>>(kin, vin, ktmp, vtmp, n);
+// The middle merge: every span of 32 tiles.
+template <int kTile>
+__global__ __launch_bounds__(kSpanThreads) void k_merge_spans(const uint64_t* __restrict__ kin,
+                                                              const uint32_t* __restrict__ vin,
+                                                              uint64_t* __restrict__ kout,
+                                                              uint32_t* __restrict__ vout, int n) {
+  asm volatile("griddepcontrol.wait;" : "+l"(kin), "+l"(vin)::"memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  int place;
+  uint64_t key;
+  uint32_t val;
+  if (!span_merge_rank<kTile, 32 * kTile>(kin, vin, n, place, key, val)) return;
+  kout[place] = key;
+  vout[place] = val;
+}
+
+// A merge as a dependent of the kernel before it on the stream.
+void launch_dependent(void (*kernel)(const uint64_t*, const uint32_t*, uint64_t*, uint32_t*, int), int blocks,
+                      int threads, const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, int n,
+                      cudaStream_t st) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(merge_blocks(n));
-  cfg.blockDim = dim3(merge_threads(n));
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, BH_TILE_KERNEL(k_merge_pairs, n, false), (const uint64_t*)ktmp, (const uint32_t*)vtmp,
-                     kout, vout, n);
+  cudaLaunchKernelEx(&cfg, kernel, kin, vin, kout, vout, n);
+}
+
+auto spans_kernel(const TileShape& sh) {
+  return sh.tile == kTileSmall ? k_merge_spans<kTileSmall> : k_merge_spans<kTileSpan>;
+}
+
+// Sorts n pairs by tiles into kout / vout (which may be kin / vin); returns the number of launches.
+int launch_tile_sort(const uint64_t* kin, const uint32_t* vin, uint64_t* ktmp, uint32_t* vtmp, uint64_t* kout,
+                     uint32_t* vout, int n, cudaStream_t st) {
+  const TileShape sh = pairs_shape(n);
+  uint64_t* kt = sh.span ? kout : ktmp;  // with spans one more change of buffers: the tiles start in the output
+  uint32_t* vt = sh.span ? vout : vtmp;
+  BH_TILE_KERNEL(k_tile_pairs, sh)<<<sh.tile_blocks(), sh.tile, 0, st>>>(kin, vin, kt, vt, n);
+  if (sh.span) launch_dependent(spans_kernel(sh), sh.merge_blocks(), kSpanThreads, kt, vt, ktmp, vtmp, n, st);
+  launch_dependent(sh.run() == 32 * kTileSmall ? k_merge_pairs<32 * kTileSmall, false> : BH_MERGE_KERNEL(k_merge_pairs, sh),
+                   sh.merge_blocks(), sh.merge_threads(), ktmp, vtmp, kout, vout, n, st);
+  return sh.span ? 3 : 2;
 }
 
 }  // namespace
 
-// Stages from the keys to the tree order of one step, radix sort / two-launch sort (us, theta 1.2, leaf
-// capacity 8): 1 000 bodies 116 / 36; 4 444 147 / 41; 16 384 155 / 49; 65 536 172 / 88; 98 304 171 / 139;
-// 131 072 176 / 178; 262 144 192 / 512.
-int tile_sort_max() { return 98304; }
+// Stages from the keys to the tree order of one step (us, theta 1.2, leaf capacity 8), radix sort / tiles /
+// tiles on a new state, whose bodies are in random order: 1 000 bodies 116 / 27 / -; 16 384 155 / 46 / -;
+// 65 536 167 / 88 / 106; 98 304 173 / 100 / 125; 131 072 180 / 117 / 141; 163 840 180 / 137 / 175; 200 000
+// 182 / 156 / 209; 262 144 194 / 198 / 271.
+int tile_sort_max() { return 163840; }
+
+// The middle merge of the pairs in keys[1] / vals[1], inside a step.
+void launch_merge_spans(bh_ctx* c, int n, uint64_t* kout, uint32_t* vout) {
+  c->launches += 1;
+  const TileShape sh = step_shape(n);
+  spans_kernel(sh)<<<sh.merge_blocks(), kSpanThreads, 0, c->stream>>>(c->keys[1], c->vals[1], kout, vout, n);
+}
 
 int sort_max_tiles(size_t n) { return (int)((n + kTile - 1) / kTile); }
 
@@ -330,8 +369,7 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
   if (n <= 1) return;
   if (n <= tile_sort_max() && first_pass == 0 && npasses == kPasses) {
     // the result goes back to keys_in / vals_in, as after the eight digit passes
-    c->launches += 2;
-    launch_tile_sort(keys_in, vals_in, keys_tmp, vals_tmp, keys_in, vals_in, n, st);
+    c->launches += launch_tile_sort(keys_in, vals_in, keys_tmp, vals_tmp, keys_in, vals_in, n, st);
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);

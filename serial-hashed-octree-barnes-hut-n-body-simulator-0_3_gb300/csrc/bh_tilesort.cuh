@@ -1,16 +1,17 @@
-// Two-launch stable sort of up to kTileSortMax (u64 key, u32 value) pairs, as building blocks that
-// the stage kernels fuse with what makes the keys and with what consumes the sorted order.
+// Stable sort of up to tile_sort_max() (u64 key, u32 value) pairs in two launches, or three, as building
+// blocks that the stage kernels fuse with what makes the keys and with what consumes the sorted order.
 //
-//   tile:  a block sorts 128 or 512 pairs. Each warp ranks its 32 keys by comparing them all (a
+//   tile:  a block sorts 128, 256 or 512 pairs. Each warp ranks its 32 keys by comparing them all (a
 //          broadcast read per comparison), which gives 4 or 16 sorted runs in shared memory; a
 //          key's place in the tile is its place in its run plus, by binary search, its place in
 //          the other runs.
-//   merge: a key's final place is its place in its tile plus, by binary search, its place in every
-//          other tile. A block takes 32 keys and its eight warps share the tiles.
+//   spans: (larger sorts) the same as the merge within every 32 tiles, a warp for 32 keys.
+//   merge: a key's final place is its place in its tile or span plus, by binary search, its place in
+//          every other one. A block takes 32 keys and its warps share the tiles.
 //
 // Equal keys count when they stand in an earlier run or tile, so the sort is stable. The radix sort's
-// eight digit passes are a chain of 10 dependent launches, this is two; its work grows with n^2 over
-// the tile, which sets the limit.
+// eight digit passes are a chain of 10 dependent launches, this is two or three; its work grows with
+// n^2 over the tile or span, which sets the limits.
 //
 // Segments (ensembles): every system keeps its slot range, and pairs are ordered by (system, key).
 // Slots are grouped by system, so system s fills the same places of a tile before and after the
@@ -26,6 +27,18 @@ constexpr int kTileSmall = 128, kTileLarge = 512;
 // 1 000 bodies 36 / 27, 4 444 38 / 31, 16 384 47 / 46, 32 768 61 / 63, 65 536 86 / 137.
 constexpr int kTileSmallMax = 16384;
 constexpr int kMergeParts = 8;  // warps of a merge block, at most
+// Larger sorts take a middle launch that merges spans of 32 tiles (a warp for every 32 keys), and the
+// final merge takes the spans: a key is searched in 32 + n / span runs instead of n / tile.
+constexpr int kTileSpan = 256;
+constexpr int kSpanThreads = 128;
+// A step's sorts up to here stay at two launches. Whole steps with two / three launches (us, theta 1.2,
+// leaf capacity 8): 32 768 bodies 183 / 195, 49 152 218 / 225, 65 536 242 / 242, 80 000 289 / 272, 98 304
+// 326 / 293, 163 840 495 / 380.
+constexpr int kTwoLaunchMax = 65536;
+// Pairs in random order gain sooner, as fewer tiles agree. Two launches / tiles of 128 / tiles of 256 (us):
+// 24 000 35 / 41 / 45, 40 001 57 / 47 / 53, 65 536 89 / 53 / 51, 98 304 156 / 70 / 64.
+constexpr int kTwoLaunchPairsMax = 32768;
+constexpr int kSpanSmallMax = 65536;
 
 // Sorted order of (system, key); without segments the systems are all 0 and the compiler drops them.
 template <bool kSeg>
@@ -86,12 +99,65 @@ __device__ __forceinline__ int tile_count(const uint64_t* __restrict__ kin, int 
   return p;
 }
 
+// How many of the keys of [o0, o1) outside tile `own` sort before each lane's key: this warp's share of
+// the tiles (32 at a time, from tile t0 on, `step` tiles further each time), to be added up over the
+// warps. The warp's 32 keys stand in order, kfirst to klast.
+// A lane takes a tile and finds how many of its keys come before the first and before the last of the
+// 32. Where the two agree (most tiles, once the bodies are in the previous step's order) that is the
+// count for all 32 keys; the others are searched between the two, a key per lane.
+template <int kTileKeys>
+__device__ __forceinline__ int tile_counts(const uint64_t* __restrict__ kin, int o0, int o1, int own, int t0, int step32,
+                                           uint64_t key, uint64_t kfirst, uint64_t klast) {
+  const int lane = threadIdx.x & 31, tlast = (o1 - 1) / kTileKeys;
+  int cnt = 0, shared_cnt = 0;  // shared_cnt: this lane's tiles, keys before all 32
+  for (; t0 <= tlast; t0 += step32) {
+    const int tile = t0 + lane;
+    int lo = max(o0, tile * kTileKeys), len = min(o1, (tile + 1) * kTileKeys) - lo, c0 = 0, c1 = 0;
+    if (tile <= tlast && tile != own) {
+      for (int step = kTileKeys; step > 0; step >>= 1) {  // the two searches side by side
+        const bool f0 = c0 + step <= len, f1 = c1 + step <= len;
+        const uint64_t k0 = kin[lo + (f0 ? c0 + step - 1 : 0)], k1 = kin[lo + (f1 ? c1 + step - 1 : 0)];
+        if (f0 && (tile < own ? k0 <= kfirst : k0 < kfirst)) c0 += step;
+        if (f1 && (tile < own ? k1 <= klast : k1 < klast)) c1 += step;
+      }
+      shared_cnt += c0;
+    }
+    uint32_t open = __ballot_sync(0xffffffffu, c1 > c0);
+    lo += c0;
+    len = c1 - c0;
+    while (open) {  // four tiles' searches in flight
+      constexpr int kFlight = 4;
+      int clo[kFlight], clen[kFlight], p[kFlight], longest = 0;
+      bool earlier[kFlight];
+#pragma unroll
+      for (int q = 0; q < kFlight; ++q) {
+        const int src = open ? __ffs(open) - 1 : 0;
+        clo[q] = __shfl_sync(0xffffffffu, lo, src);
+        if (!open) clo[q] = 0;  // an empty search reads key 0
+        clen[q] = open ? __shfl_sync(0xffffffffu, len, src) : 0;
+        earlier[q] = t0 + src < own;
+        open &= open - 1;
+        p[q] = 0;
+        longest = max(longest, clen[q]);
+      }
+      for (int step = 1 << (31 - __clz(longest)); step > 0; step >>= 1) {
+#pragma unroll
+        for (int q = 0; q < kFlight; ++q) {
+          const bool fits = p[q] + step <= clen[q];
+          const uint64_t k = kin[clo[q] + (fits ? p[q] + step - 1 : 0)];
+          if (fits && (earlier[q] ? k <= key : k < key)) p[q] += step;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kFlight; ++q) cnt += p[q];
+    }
+  }
+  return cnt + __reduce_add_sync(0xffffffffu, shared_cnt);
+}
+
 // Final places of the block's 32 keys (tile-sorted slots 32 blockIdx.x ..): true in the lanes of the
-// first warp that hold a key, with its place, key and value. All threads call it.
-// A warp takes 32 tiles at once, a tile per lane, and finds how many of its keys come before the
-// block's first and before its last key. Where the two agree (most tiles, once the bodies are
-// in the previous step's order) that is the count for all 32 keys; the others are searched between
-// the two, a key per lane.
+// first warp that hold a key, with its place, key and value. All threads call it; the block's warps
+// share the tiles.
 // kSeg: pairs ordered by (system, key), off the systems' slot ranges, body_sys each slot's system. A
 // slot's system is that of every pair the tile sort may put there.
 template <int kTileKeys, bool kSeg>
@@ -116,51 +182,7 @@ __device__ __forceinline__ bool tile_merge_rank(const uint64_t* __restrict__ kin
   }
   int cnt = 0;
   if (same) {
-    const int tfirst = o0 / kTileKeys, tlast = (o1 - 1) / kTileKeys;
-    int shared_cnt = 0;  // this lane's tiles: keys before all of the block's
-    for (int t0 = tfirst + part * 32; t0 <= tlast; t0 += parts * 32) {
-      const int tile = t0 + lane;
-      int lo = max(o0, tile * kTileKeys), len = min(o1, (tile + 1) * kTileKeys) - lo, c0 = 0, c1 = 0;
-      if (tile <= tlast && tile != own) {
-        for (int step = kTileKeys; step > 0; step >>= 1) {  // the two searches side by side
-          const bool f0 = c0 + step <= len, f1 = c1 + step <= len;
-          const uint64_t k0 = kin[lo + (f0 ? c0 + step - 1 : 0)], k1 = kin[lo + (f1 ? c1 + step - 1 : 0)];
-          if (f0 && (tile < own ? k0 <= kfirst : k0 < kfirst)) c0 += step;
-          if (f1 && (tile < own ? k1 <= klast : k1 < klast)) c1 += step;
-        }
-        shared_cnt += c0;
-      }
-      uint32_t open = __ballot_sync(0xffffffffu, c1 > c0);
-      lo += c0;
-      len = c1 - c0;
-      while (open) {  // four tiles' searches in flight
-        constexpr int kFlight = 4;
-        int clo[kFlight], clen[kFlight], p[kFlight], longest = 0;
-        bool earlier[kFlight];
-#pragma unroll
-        for (int q = 0; q < kFlight; ++q) {
-          const int src = open ? __ffs(open) - 1 : 0;
-          clo[q] = __shfl_sync(0xffffffffu, lo, src);
-          if (!open) clo[q] = 0;  // an empty search reads key 0
-          clen[q] = open ? __shfl_sync(0xffffffffu, len, src) : 0;
-          earlier[q] = t0 + src < own;
-          open &= open - 1;
-          p[q] = 0;
-          longest = max(longest, clen[q]);
-        }
-        for (int step = 1 << (31 - __clz(longest)); step > 0; step >>= 1) {
-#pragma unroll
-          for (int q = 0; q < kFlight; ++q) {
-            const bool fits = p[q] + step <= clen[q];
-            const uint64_t k = kin[clo[q] + (fits ? p[q] + step - 1 : 0)];
-            if (fits && (earlier[q] ? k <= key : k < key)) p[q] += step;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < kFlight; ++q) cnt += p[q];
-      }
-    }
-    cnt += __reduce_add_sync(0xffffffffu, shared_cnt);
+    cnt = tile_counts<kTileKeys>(kin, o0, o1, own, o0 / kTileKeys + part * 32, parts * 32, key, kfirst, klast);
   } else {  // several systems among the block's keys: each lane searches its own system's tiles
     const int tfirst = __reduce_min_sync(0xffffffffu, o0 / kTileKeys);
     const int tlast = __reduce_max_sync(0xffffffffu, (o1 - 1) / kTileKeys);
@@ -178,19 +200,70 @@ __device__ __forceinline__ bool tile_merge_rank(const uint64_t* __restrict__ kin
   return true;
 }
 
-// Tile size for n keys (both launches of a sort), and the launches' shapes.
-inline int tile_keys(int n) { return n <= kTileSmallMax ? kTileSmall : kTileLarge; }
-inline int tile_blocks(int n) { return (n + tile_keys(n) - 1) / tile_keys(n); }
-inline int merge_blocks(int n) { return (n + 31) / 32; }
-// a warp for every 32 tiles, up to eight
-inline int merge_threads(int n) {
-  const int parts = (tile_blocks(n) + 31) / 32;
-  return 32 * (parts < kMergeParts ? parts : kMergeParts);
+// The same with a warp for every 32 keys, for merges of about 32 tiles: within spans of kSpanKeys keys
+// (0: over all n). No barrier; whole warps return early.
+template <int kTileKeys, int kSpanKeys>
+__device__ __forceinline__ bool span_merge_rank(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                                int n, int& place, uint64_t& key, uint32_t& val) {
+  const int lane = threadIdx.x & 31;
+  const int b0 = (int)(blockIdx.x * blockDim.x + threadIdx.x - lane), i = b0 + lane, own = b0 / kTileKeys;
+  if (b0 >= n) return false;
+  const int last = min(31, n - 1 - b0);
+  key = kin[min(i, n - 1)];
+  const uint64_t kfirst = __shfl_sync(0xffffffffu, key, 0), klast = __shfl_sync(0xffffffffu, key, last);
+  const int o0 = kSpanKeys ? b0 / kSpanKeys * kSpanKeys : 0, o1 = kSpanKeys ? min(n, o0 + kSpanKeys) : n;
+  const int cnt = tile_counts<kTileKeys>(kin, o0, o1, own, o0 / kTileKeys, 32, key, kfirst, klast);
+  if (lane > last) return false;
+  place = o0 + (i - own * kTileKeys) + cnt;
+  val = vin[i];
+  return true;
 }
 
-// Launches kernel<tile size, segments> with the tile of n keys.
-#define BH_TILE_KERNEL(kernel, n, seg)                                                      \
-  (tile_keys(n) == kTileSmall ? ((seg) ? kernel<kTileSmall, true> : kernel<kTileSmall, false>) \
-                              : ((seg) ? kernel<kTileLarge, true> : kernel<kTileLarge, false>))
+// The final merge's places: of tiles, by blocks that share them, or of merged spans, a warp per 32 keys.
+template <int kTileKeys, bool kSeg>
+__device__ __forceinline__ bool merge_rank(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                           const uint16_t* __restrict__ body_sys, const uint32_t* __restrict__ off,
+                                           int n, int& place, uint64_t& key, uint32_t& val) {
+  if (kTileKeys > kTileLarge) return span_merge_rank<kTileKeys, 0>(kin, vin, n, place, key, val);
+  return tile_merge_rank<kTileKeys, kSeg>(kin, vin, body_sys, off, n, place, key, val);
+}
+
+// The launches of a sort of n keys: tiles of `tile` keys, merged in spans of `span` keys (0: not), then
+// runs of `run()` keys into the result.
+struct TileShape {
+  int n, tile, span;
+  int run() const { return span ? span : tile; }
+  int tile_blocks() const { return (n + tile - 1) / tile; }
+  // without spans a warp for every 32 tiles, up to eight, share 32 keys
+  int merge_threads() const {
+    const int parts = (tile_blocks() + 31) / 32;
+    return span ? kSpanThreads : 32 * (parts < kMergeParts ? parts : kMergeParts);
+  }
+  int merge_blocks() const { return span ? (n + kSpanThreads - 1) / kSpanThreads : (n + 31) / 32; }
+};
+
+// In a step the keys are nearly in order. Ensembles (seg) never merge spans: their systems are short.
+inline TileShape step_shape(int n, bool seg = false) {
+  if (!seg && n > kTwoLaunchMax) return {n, kTileSpan, 32 * kTileSpan};
+  return {n, n <= kTileSmallMax ? kTileSmall : kTileLarge, 0};
+}
+// Pairs in any order.
+inline TileShape pairs_shape(int n) {
+  if (n > kSpanSmallMax) return {n, kTileSpan, 32 * kTileSpan};
+  if (n > kTwoLaunchPairsMax) return {n, kTileSmall, 32 * kTileSmall};
+  return {n, n <= kTileSmallMax ? kTileSmall : kTileLarge, 0};
+}
+
+// The kernel instance of a shape's tiles and of its final merge.
+#define BH_TILE_KERNEL(kernel, shape)                      \
+  ((shape).tile == kTileSmall  ? kernel<kTileSmall, false> \
+   : (shape).tile == kTileSpan ? kernel<kTileSpan, false>  \
+                               : kernel<kTileLarge, false>)
+#define BH_TILE_KERNEL_SEG(kernel, shape) \
+  ((shape).tile == kTileSmall ? kernel<kTileSmall, true> : kernel<kTileLarge, true>)
+#define BH_MERGE_KERNEL(kernel, shape)                      \
+  ((shape).run() == kTileSmall   ? kernel<kTileSmall, false> \
+   : (shape).run() == kTileLarge ? kernel<kTileLarge, false> \
+                                 : kernel<32 * kTileSpan, false>)
 
 }  // namespace bh

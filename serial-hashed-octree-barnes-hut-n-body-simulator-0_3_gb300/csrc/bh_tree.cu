@@ -453,7 +453,7 @@ __global__ __launch_bounds__(kThreads) void k_gather_kd_treekey(
   tidx[j] = (uint32_t)j;
 }
 
-// ---- systems small enough for the two-launch sort (tile_sort_max): the stages around it in its kernels
+// ---- systems small enough to sort by tiles (tile_sort_max): the stages around the sort in its kernels
 
 // Morton keys, tile-sorted with their slots (kSeg: by the slots' systems first).
 template <int kTile, bool kSeg>
@@ -478,7 +478,7 @@ __global__ __launch_bounds__(32 * kMergeParts) void k_merge_kd(
   int j;
   uint64_t key;
   uint32_t i;
-  if (!tile_merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, j, key, i)) return;
+  if (!merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, j, key, i)) return;
   float4 p = pin[i], v = velin[i];
   kick_drift(p, v, acc[acc_follows_body ? i : (uint32_t)j], dt, half_dt);
   pout[j] = p;
@@ -539,7 +539,7 @@ __global__ __launch_bounds__(32 * kMergeParts) void k_merge_tree(const uint64_t*
   int r;
   uint64_t key;
   uint32_t slot;
-  if (!tile_merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, r, key, slot)) return;
+  if (!merge_rank<kTile, kSeg>(kin, vin, body_sys, off, n, r, key, slot)) return;
   tkey[r] = key;
   tslot[r] = slot;
   tpos[r] = pos[slot];
@@ -1816,39 +1816,53 @@ void launch_gather_kd_treekey(bh_ctx* c, const uint32_t* perm, int n, const floa
         batch ? c->body_sys : nullptr, pout, vout, tkeys, tidx);
 }
 
-// The stages of a step up to the tree order, for systems that sort in two launches. The tile-sorted
-// pairs pass through keys[1] / vals[1].
+// The stages of a step up to the tree order, for systems that sort by tiles. The tile-sorted pairs pass
+// through keys[1] / vals[1]; merged spans, where the sort has them, through arrays that are free until
+// the tree order (tkey / tslot) and the build (nkey, vals[0]).
 void launch_morton_tiles(bh_ctx* c, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_morton_tiles, n, batch)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
+  const TileShape sh = step_shape(n, batch);
+  (batch ? BH_TILE_KERNEL_SEG(k_morton_tiles, sh)
+         : BH_TILE_KERNEL(k_morton_tiles, sh))<<<sh.tile_blocks(), sh.tile, 0, c->stream>>>(
       pos, n, batch ? c->sys_geom : c->geom, c->body_sys, c->keys[1], c->vals[1]);
+  if (sh.span) launch_merge_spans(c, n, c->tkey, c->tslot);
 }
 
 void launch_merge_kd(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, int acc_follows_body,
                      float dt, float4* pout, float4* vout, uint64_t* kout, uint64_t* ktree, bool batch) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_merge_kd, n, batch)<<<merge_blocks(n), merge_threads(n), 0, c->stream>>>(
-      c->keys[1], c->vals[1], n, pin, vin, acc, acc_follows_body, dt, 0.5f * dt, batch ? c->sys_geom : c->geom,
+  const TileShape sh = step_shape(n, batch);
+  (batch ? BH_TILE_KERNEL_SEG(k_merge_kd, sh)
+         : BH_MERGE_KERNEL(k_merge_kd, sh))<<<sh.merge_blocks(), sh.merge_threads(), 0, c->stream>>>(
+      sh.span ? c->tkey : c->keys[1], sh.span ? c->tslot : c->vals[1], n, pin, vin, acc, acc_follows_body, dt,
+      0.5f * dt, batch ? c->sys_geom : c->geom,
       c->body_sys, c->sys_off, pout, vout, kout, ktree);
 }
 
 void launch_kd_tiles(bh_ctx* c, int n, const float4* pin, const float4* vin, const float4* acc, float dt, float4* pout,
                      float4* vout) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_kd_tiles, n, false)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
+  const TileShape sh = step_shape(n);
+  BH_TILE_KERNEL(k_kd_tiles, sh)<<<sh.tile_blocks(), sh.tile, 0, c->stream>>>(
       pin, vin, acc, c->tslot, n, dt, 0.5f * dt, c->geom, pout, vout, c->keys[1], c->vals[1]);
+  if (sh.span) launch_merge_spans(c, n, c->nkey, c->vals[0]);
 }
 
 void launch_tree_tiles(bh_ctx* c, const uint64_t* ktree, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_tree_tiles, n, batch)<<<tile_blocks(n), tile_keys(n), 0, c->stream>>>(
+  const TileShape sh = step_shape(n, batch);
+  (batch ? BH_TILE_KERNEL_SEG(k_tree_tiles, sh)
+         : BH_TILE_KERNEL(k_tree_tiles, sh))<<<sh.tile_blocks(), sh.tile, 0, c->stream>>>(
       ktree, pos, n, c->geom, c->body_sys, c->keys[1], c->vals[1]);
+  if (sh.span) launch_merge_spans(c, n, c->nkey, c->vals[0]);
 }
 
 void launch_merge_tree(bh_ctx* c, const float4* pos, int n, bool batch) {
   c->launches += 1;
-  BH_TILE_KERNEL(k_merge_tree, n, batch)<<<merge_blocks(n), merge_threads(n), 0, c->stream>>>(
-      c->keys[1], c->vals[1], n, pos, c->body_sys, c->sys_off, c->tkey, c->tslot, c->tpos);
+  const TileShape sh = step_shape(n, batch);
+  (batch ? BH_TILE_KERNEL_SEG(k_merge_tree, sh)
+         : BH_MERGE_KERNEL(k_merge_tree, sh))<<<sh.merge_blocks(), sh.merge_threads(), 0, c->stream>>>(
+      sh.span ? c->nkey : c->keys[1], sh.span ? c->vals[0] : c->vals[1], n, pos, c->body_sys, c->sys_off, c->tkey, c->tslot, c->tpos);
 }
 
 void launch_kick_drift(bh_ctx* c, float4* pos, float4* vel, const float4* acc, int n, float dt, int drift) {
