@@ -90,6 +90,12 @@ struct Acc {
     cz = (t - sz) - y;
     sz = t;
   }
+  // x to the first sum, its rounding error to the first compensation (two-sum, whichever is larger)
+  __device__ __forceinline__ void add_exactly(float x) {
+    const float t = sx + x, b = t - sx;
+    cx -= (sx - (t - b)) + (x - b);
+    sx = t;
+  }
 };
 
 // Interaction recording for the adjoint: where the flushed buffers go, and the current group.
@@ -233,7 +239,9 @@ __device__ __forceinline__ void eval_points(Smem& s, int cnt, const WalkNode* __
 }
 
 // The potential's terms (diagnostics): M / D + d.Q.d / (2 D^5) of a cell, m / D of a point at another
-// position than the body's. phi = -sum, every term added to a compensated per-lane sum (acc.sx).
+// position than the body's. phi = -sum, summed with every rounding error kept and rounded once at
+// the end, so that it does not depend on the order in which a group meets its cells and bodies. The terms
+// don't either: the softening is added first to a body's D^2, last to a node's, whoever they go with.
 template <bool kCells, int kGroup, class Smem>
 __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode* __restrict__ nodes,
                                                const float4* __restrict__ tpos, int lane, float px, float py, float pz,
@@ -255,7 +263,9 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
       v2.w = __uint_as_float(s.pt_mask[lane]);
       if (e >= 0) {
         v = __ldg(tpos + e);
+        v2.x = eps2;
       } else {
+        v2.y = eps2;
         const WalkNode* nd = nodes + (-e - 1);
         const float4 mac = __ldg(&nd->mac);
         v = make_float4(mac.x, mac.y, mac.z, __ldg(&nd->mq.x));
@@ -271,8 +281,8 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
     const int j = r + slot;
     const float4 c0 = s.st0[j], c2 = s.st2[j];
     const float dx = c0.x - px, dy = c0.y - py, dz = c0.z - pz;
-    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float rinv = rsqrtf(d2 + eps2);
+    const float d2 = fmaf(dx, dx, fmaf(dy, dy, kCells ? dz * dz : fmaf(dz, dz, c2.x)));
+    const float rinv = rsqrtf(d2 + (kCells ? eps2 : c2.y));
     bool take = (__float_as_uint(c2.w) & lanebit) != 0u;
     float term;
     if (kCells) {
@@ -287,10 +297,11 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
       term = c0.w * rinv;
       take = take && !((dx == 0.f) & (dy == 0.f) & (dz == 0.f));
     }
-    const float y = (take ? -term : 0.f) - acc.cx, t = acc.sx + y;
-    acc.cx = (t - acc.sx) - y;
-    acc.sx = t;
+    acc.add_exactly(take ? -term : 0.f);
   }
+  const float t = acc.sx - acc.cx;  // the errors stay below half an ulp of the sum
+  acc.cx = (t - acc.sx) + acc.cx;
+  acc.sx = t;
 }
 
 // Moves buffer entries [32, n) to [0, n - 32) after the first 32 were evaluated.
@@ -684,7 +695,15 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
     }
     if (ncell > 0) run_cells(ncell);
     if (npt > 0) run_points(npt);
-    if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
+    if (kPot) {  // the slots' sums of each body
+#pragma unroll
+      for (int o = kGroup; o < 32; o <<= 1) {
+        const float os = __shfl_xor_sync(0xffffffffu, acc.sx, o), oc = __shfl_xor_sync(0xffffffffu, acc.cx, o);
+        acc.cx += oc;
+        acc.add_exactly(os);
+      }
+      acc.sx -= acc.cx;
+    } else if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
 #pragma unroll
       for (int o = kGroup; o < 32; o <<= 1) {
         const float ox = __shfl_xor_sync(0xffffffffu, acc.sx, o), oy = __shfl_xor_sync(0xffffffffu, acc.sy, o),
