@@ -96,10 +96,11 @@ typedef struct bh_stats {
   double ms_step;          /* whole steps, first to last kernel */
   double ms_bounds;
   double ms_morton;
-  double ms_sort;          /* Morton-key sort of the bodies */
+  double ms_sort;          /* Morton-key sort of the bodies; of systems sorted by tiles (up to 163 840
+                              bodies) with the work of the next line, which the sort then does */
   double ms_kick_drift;    /* gather into sorted order + first half-kick + drift + tree keys */
   double ms_sort_tree;     /* tree-key sort */
-  double ms_build;         /* node discovery + hash table */
+  double ms_build;         /* node discovery */
   double ms_upsweep;
   double ms_walk;          /* tree walk + force (+ second half-kick inside bh_step) */
   uint64_t n_nodes;
@@ -259,7 +260,7 @@ bh_status bh_measure_fp32_peak(bh_ctx* ctx, double* tflops);
  * BH_SORT_STATIC_MAX_KEYS (larger n returns BH_ERR_INVALID_ARG). Sorts stably by the full
  * 64-bit key (the same permutation as bh_sort_bodies) into keys_out / vals_out; the inputs
  * are left unchanged; asynchronous on `stream` (a cudaStream_t, NULL for the legacy default
- * stream) on the current device. status_out (optional, device memory) is set to 0: the sort's two
+ * stream) on the current device. status_out (optional, device memory) is set to 0: the sort's
  * launches have no device-side wait that could give up.
  * The first call on each device looks up the scratch array's device address, so make it before
  * any stream capture on that device. The address is kept for the life of the process: after a
