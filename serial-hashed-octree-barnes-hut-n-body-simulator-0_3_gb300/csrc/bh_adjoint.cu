@@ -439,19 +439,21 @@ bh_status capture_tree(bh_ctx* c, TapeSlot& t) {
   return BH_OK;
 }
 
-// Records the step (or the initial force when step == false) into slot t, growing the chunk
-// capacity and redoing it when the tape overflows. The state is restored by the caller-provided
-// snapshot before a redo (the step is transactional through the ping-pong buffers).
-bh_status record_into(bh_ctx* c, AdjState* a, TapeSlot& t, bool step) {
+// Records the step (or the force at the current positions when step == false) into slot t, of at least
+// chunk_cap chunks. On BH_ERR_OVERFLOW_TAPE the walk has run to its end: the accelerations are the new
+// ones, so a step cannot be redone from here.
+bh_status record_into(bh_ctx* c, AdjState* a, TapeSlot& t, size_t chunk_cap, bool step) {
+  BH_TRY(ensure_slot(t, c->n, c->node_cap, chunk_cap));
+  BH_TRY(step ? fixed_step(c, a->prm, &t) : force_at_current(c, a->prm, &t));
+  return capture_tree(c, t);
+}
+
+// The force at the current positions (which it does not change) with a tape grown to hold it.
+bh_status record_force(bh_ctx* c, AdjState* a, TapeSlot& t) {
   for (;;) {
-    BH_TRY(ensure_slot(t, c->n, c->node_cap, a->chunk_cap));
-    const bh_status s = step ? fixed_step(c, a->prm, &t) : force_at_current(c, a->prm, &t);
-    if (s == BH_ERR_OVERFLOW_TAPE) {
-      a->chunk_cap *= 2;
-      continue;
-    }
-    BH_TRY(s);
-    return capture_tree(c, t);
+    const bh_status s = record_into(c, a, t, a->chunk_cap, false);
+    if (s != BH_ERR_OVERFLOW_TAPE) return s;
+    a->chunk_cap *= 2;
   }
 }
 
@@ -494,6 +496,24 @@ bh_status restore_checkpoint(bh_ctx* c, AdjState* a, int k) {
   cudaMemcpyAsync(c->vel[0], ck_ptr(a, k, 1), bytes, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(c->acc, ck_ptr(a, k, 2), bytes, cudaMemcpyDeviceToDevice, c->stream);
   return last_launch();
+}
+
+// The steps of segment seg, from its checkpoint, recorded into the first `len` tape slots. When a step fills
+// its tape, the whole segment is recorded again, with larger slots from that step on.
+bh_status record_segment(bh_ctx* c, AdjState* a, int seg, int len) {
+  int enough = 0;  // slots that held their step
+  for (;;) {
+    BH_TRY(restore_checkpoint(c, a, seg));
+    bh_status s = BH_OK;
+    for (int k = 0; k < len; ++k) {
+      TapeSlot& t = a->tape[k];
+      s = record_into(c, a, t, k < enough ? t.chunk_cap : a->chunk_cap, true);
+      if (s != BH_OK) break;
+      enough = std::max(enough, k + 1);
+    }
+    if (s != BH_ERR_OVERFLOW_TAPE) return s;
+    a->chunk_cap *= 2;
+  }
 }
 
 }  // namespace
@@ -567,7 +587,7 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
   cudaEvent_t e0 = c->stage_ev[0], e1 = c->stage_ev[1];
   const uint64_t launches0 = c->launches;
   cudaEventRecord(e0, c->stream);
-  BH_TRY(record_into(c, a, a->tape[0], false));
+  BH_TRY(record_force(c, a, a->tape[0]));
   a->chunk_cap = std::max<size_t>(a->chunk_cap, (size_t)(a->tape[0].nchunks * 1.5) + 1024);
   const size_t bytes = sizeof(float4) * c->n;
   for (int s = 0; s < nsteps; ++s) {
@@ -627,8 +647,7 @@ bh_status bh_step_backward(bh_ctx* c, const float* dl_dx4, const float* dl_dv4, 
   const int nseg = (a->nsteps + every - 1) / every;
   for (int seg = nseg - 1; seg >= 0; --seg) {
     const int s0 = seg * every, s1 = std::min(s0 + every, a->nsteps);
-    BH_TRY(restore_checkpoint(c, a, seg));
-    for (int t = 0; t < s1 - s0; ++t) BH_TRY(record_into(c, a, a->tape[t], true));
+    BH_TRY(record_segment(c, a, seg, s1 - s0));
     for (int stp = s1 - 1; stp >= s0; --stp) {
       const TapeSlot& t = a->tape[stp - s0];
       k_adj_abar<<<grid_for(n), kThreads, 0, c->stream>>>(a->vbar, a->carry, h, n, a->abar);
@@ -639,7 +658,7 @@ bh_status bh_step_backward(bh_ctx* c, const float* dl_dx4, const float* dl_dv4, 
   }
   // a(x_0): the carry is its adjoint
   BH_TRY(restore_checkpoint(c, a, 0));
-  BH_TRY(record_into(c, a, a->tape[0], false));
+  BH_TRY(record_force(c, a, a->tape[0]));
   cudaMemcpyAsync(a->abar, a->carry, bytes, cudaMemcpyDeviceToDevice, c->stream);
   BH_TRY(vjp(c, a, a->tape[0]));
   if (grad_x4) cudaMemcpyAsync(grad_x4, a->xbar, bytes, cudaMemcpyDeviceToHost, c->stream);
