@@ -98,6 +98,7 @@ void clear_device_flags(bh_ctx* c) {
 size_t initial_node_cap(size_t n) { return std::max<size_t>(2 * n + 64, 1024); }
 
 void launch_tree_order(bh_ctx* c, const float4* pos, int n) {
+  if (n <= 0) return;  // an empty state has an empty order
   if (n <= tile_sort_max()) {
     bh::launch_tree_tiles(c, nullptr, pos, n);
     bh::launch_merge_tree(c, pos, n);
