@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "bh_internal.cuh"
 #include "bh_tilesort.cuh"
@@ -1260,11 +1261,20 @@ __device__ __forceinline__ void write_multipole(int node, int part, const Moment
   *dst = v;
 }
 
-// Edge^2 of a node: the root edge squared in FP64 and rounded, times 4^-depth (exact).
+__device__ __noinline__ float node_edge2_exact(double root_edge, int d) {
+  const double edge = ldexp(root_edge, -d);
+  return __double2float_rn(__dmul_rn(edge, edge));
+}
+
+// Edge^2 of a node, the FP64 square rounded to float. Where the root's square and the node's are both
+// normal floats, that is the rounded root's square times 4^-depth (exact); otherwise (the square of an edge
+// above 2^64 is no float, although those of the nodes below may be) it is formed in FP64.
 __device__ __forceinline__ float node_edge2(uint64_t key, int first, const Geom* __restrict__ g,
                                             const uint16_t* __restrict__ body_sys) {
   const int d = (63 - __clzll((long long)key)) / 3;
-  return ldexpf(body_sys ? g[body_sys[first]].tedge2 : g->tedge2, -2 * d);
+  const Geom& root = body_sys ? g[body_sys[first]] : *g;
+  const float s2 = ldexpf(root.tedge2, -2 * d);
+  return s2 >= FLT_MIN && s2 <= FLT_MAX ? s2 : node_edge2_exact(root.tedge, d);
 }
 
 // A node's range as bodies, chunks and supers: bodies [first, b0) and [b1, end), chunks [c0, d0)
