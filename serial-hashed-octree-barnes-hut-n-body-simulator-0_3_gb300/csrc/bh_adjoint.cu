@@ -366,7 +366,7 @@ bh_status force_at_current(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
       launch_walk_record(c, n, (float)p.theta, (float)p.eps, c->acc, nullptr, 0.f, rec->chunks, rec->count,
                          (int)rec->chunk_cap);
     } else {
-      launch_walk(c, n, (float)p.theta, (float)p.eps, BH_MULTIPOLE_QUADRUPOLE, c->acc, nullptr, 0.f);
+      launch_walk_unrecorded(c, n, (float)p.theta, (float)p.eps, c->acc, nullptr, 0.f);
     }
     BH_TRY(last_launch());
     uint32_t e = 0;
@@ -405,7 +405,7 @@ bh_status fixed_step(bh_ctx* c, const bh_params& p, TapeSlot* rec) {
       launch_walk_record(c, n, (float)p.theta, (float)p.eps, c->acc, c->vel[nx], 0.5f * dt, rec->chunks, rec->count,
                          (int)rec->chunk_cap);
     } else {
-      launch_walk(c, n, (float)p.theta, (float)p.eps, BH_MULTIPOLE_QUADRUPOLE, c->acc, c->vel[nx], 0.5f * dt);
+      launch_walk_unrecorded(c, n, (float)p.theta, (float)p.eps, c->acc, c->vel[nx], 0.5f * dt);
     }
     BH_TRY(last_launch());
     uint32_t e = 0;

@@ -308,6 +308,8 @@ void launch_hash(bh_ctx* c);
 void launch_walk(bh_ctx* c, int n, float theta, float eps, int mode, float4* acc_slot, float4* vel_kick,
                  float half_dt, bool batch = false, float4* vel_copy = nullptr);
 void launch_lookup(bh_ctx* c, uint64_t key, int* out_index);
+void launch_walk_unrecorded(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick,
+                            float half_dt);
 void launch_walk_record(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick, float half_dt,
                         Chunk* tape, unsigned* tape_count, int tape_cap);
 void launch_fp32_peak(cudaStream_t st, float* sink, int blocks);
@@ -321,7 +323,7 @@ int walk_variants();
 WalkVariant walk_variant_info(int v, size_t n);
 // Bodies per walk group for n bodies in all (a single system, or the systems of an ensemble).
 int walk_group_size(size_t n);
-// Bodies per group of the recording walk.
+// Bodies per group of the differentiable path's walks.
 int record_group_size(size_t n);
 void launch_walk_variant(bh_ctx* c, int v, int n, float theta, float eps, float4* acc_out, bool batch);
 

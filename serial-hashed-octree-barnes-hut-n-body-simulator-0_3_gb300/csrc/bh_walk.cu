@@ -1007,8 +1007,19 @@ static void launch_walk_record_t(bh_ctx* c, int n, float theta, float eps, float
       c->counters, c->err, tape, tape_count, tape_cap);
 }
 
-// Bodies per recorded group: 16 where the force walk's groups are at most 16.
+// Bodies per group of the differentiable path: 16 where the force walk's groups are at most 16.
 int record_group_size(size_t n) { return std::min(32, std::max(16, walk_group_size(n))); }
+
+// The recording walk without its tape, for the forward pass: the same groups whatever the context's variant,
+// so that a recomputed step repeats the forward step's sums bit for bit. (Forward steps in groups of 4 or
+// 8 would walk 10 to 26% faster below 24 576 bodies, but recomputed trajectories would drift away from them.)
+void launch_walk_unrecorded(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick,
+                            float half_dt) {
+  if (n <= 0) return;
+  c->launches += 1;
+  launch_quad_default(c, n, WalkArgs{theta * theta, eps * eps, half_dt, acc_slot, vel_kick, nullptr, false},
+                      record_group_size(n));
+}
 
 // The walk of the differentiable path: quadrupole multipoles, positive softening, and every
 // flushed interaction buffer appended to `tape` (tape_count counts chunks; overflow of tape_cap
