@@ -58,6 +58,7 @@ struct AdjState {
   int nck = 0;
   size_t n = 0;
   float4* ck = nullptr;  // [nck + 1][3][n]: x, v, a at steps 0, every, 2 every, ..., then the final state
+  uint32_t* ck_order = nullptr;  // [nck][n]: the tree order that each checkpoint's next step starts from
   int final_slot = 0;
   std::vector<TapeSlot> tape;
   size_t chunk_cap = 0;
@@ -495,6 +496,9 @@ bh_status restore_checkpoint(bh_ctx* c, AdjState* a, int k) {
   cudaMemcpyAsync(c->pos[0], ck_ptr(a, k, 0), bytes, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(c->vel[0], ck_ptr(a, k, 1), bytes, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(c->acc, ck_ptr(a, k, 2), bytes, cudaMemcpyDeviceToDevice, c->stream);
+  if (a->ck_order && k != a->final_slot)
+    cudaMemcpyAsync(c->tslot, a->ck_order + (size_t)k * a->n, sizeof(uint32_t) * a->n, cudaMemcpyDeviceToDevice,
+                    c->stream);
   return last_launch();
 }
 
@@ -527,6 +531,7 @@ void adj_release(bh_ctx* c) {
   if (!a) return;
   for (auto& t : a->tape) free_slot(t);
   dfree(a->ck);
+  dfree(a->ck_order);
   dfree(a->xbar);
   dfree(a->vbar);
   dfree(a->carry);
@@ -562,6 +567,7 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
   const int nck = (nsteps + checkpoint_every - 1) / checkpoint_every;
   if (a->n != c->n || a->nck < nck) {
     dfree(a->ck);
+    dfree(a->ck_order);
     for (auto& t : a->tape) free_slot(t);
     a->tape.clear();
     dfree(a->xbar);
@@ -572,6 +578,8 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
     a->nck = 0;
     a->n = c->n;
     BH_TRY(dalloc(&a->ck, (size_t)(nck + 1) * 3 * c->n));
+    // bodies of one tree key stand in the order of the tree before (fixed_step's tile sort)
+    if (c->n <= (size_t)tile_sort_max()) BH_TRY(dalloc(&a->ck_order, (size_t)nck * c->n));
     BH_TRY(dalloc(&a->xbar, c->n));
     BH_TRY(dalloc(&a->vbar, c->n));
     BH_TRY(dalloc(&a->carry, c->n));
@@ -596,6 +604,9 @@ bh_status bh_adjoint_forward(bh_ctx* c, const bh_params* p, int nsteps, int chec
       cudaMemcpyAsync(ck_ptr(a, k, 0), c->pos[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream);
       cudaMemcpyAsync(ck_ptr(a, k, 1), c->vel[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream);
       cudaMemcpyAsync(ck_ptr(a, k, 2), c->acc, bytes, cudaMemcpyDeviceToDevice, c->stream);
+      if (a->ck_order)
+        cudaMemcpyAsync(a->ck_order + (size_t)k * c->n, c->tslot, sizeof(uint32_t) * c->n, cudaMemcpyDeviceToDevice,
+                        c->stream);
     }
     BH_TRY(fixed_step(c, a->prm, nullptr));
     if (st) {

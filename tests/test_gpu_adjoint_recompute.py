@@ -8,12 +8,28 @@ from oracle.oracle import relerr
 pytestmark = pytest.mark.gpu
 
 
-def test_gradient_does_not_depend_on_the_checkpoints(bh):
+def bodies(bh, n, dt, pairs):
+    """A sphere; or n / 2 pairs some 1e-5 apart, one body of each overtaking the other in the first step, whose
+    tree has both in one cell of the deepest level."""
+    if not pairs:
+        return bh.plummer(3, n)
+    pm, vel = bh.plummer(3, n // 2)
+    d = np.random.default_rng(3).uniform(1e-5, 3e-5, (n // 2, 3)).astype(np.float32)
+    pm2, vel2 = pm.copy(), vel.copy()
+    pm2[:, :3] -= d
+    vel2[:, :3] += d / np.float32(dt)
+    pm[:, 3] *= 0.7
+    pm2[:, 3] *= 0.3
+    return np.concatenate([pm, pm2]), np.concatenate([vel, vel2])
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+def test_gradient_does_not_depend_on_the_checkpoints(bh, pairs):
     # Up to 16 bodies under a root that is a leaf are one group and one buffer of the walk, so nothing is
     # summed in an order of chance and gradients of the same path are the same bits. With a checkpoint at
     # every step the path is the forward pass's; with fewer it is so only if each recomputed step is.
     n, nsteps, dt = 16, 50, 0.01
-    pm, vel = bh.plummer(3, n)
+    pm, vel = bodies(bh, n, dt, pairs)
     pm[:, 3] *= 100.0  # half-kicks of the size of the velocities, whose last bits then show the forces'
     prm = bh.default_params(theta=0.5, eps=0.3, dt=dt, leaf_capacity=16, multipole=1, edge_factor=1.0)
     dl = np.random.default_rng(9).normal(size=(n, 3)).astype(np.float32)
