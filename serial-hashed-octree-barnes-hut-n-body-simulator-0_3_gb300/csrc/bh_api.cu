@@ -1111,12 +1111,20 @@ bh_status batch_layout(bh_ctx* c, const uint32_t* sys_offsets, size_t nsys) {
     const uint32_t b0 = sys_offsets[s], b1 = sys_offsets[s + 1];
     largest = std::max(largest, b1 - b0);
     for (uint32_t i = b0; i < b1; ++i) bs[i] = (uint16_t)s;
-    for (uint32_t g = b0; g < b1; g += gsize)
-      groups.push_back(make_int4((int)g, (int)std::min(gsize, b1 - g), (int)s, (int)s));
   }
+  auto append_groups = [&](uint32_t size) {
+    for (size_t s = 0; s < nsys; ++s)
+      for (uint32_t g = sys_offsets[s], b1 = sys_offsets[s + 1]; g < b1; g += size)
+        groups.push_back(make_int4((int)g, (int)std::min(size, b1 - g), (int)s, (int)s));
+  };
+  append_groups(gsize);
+  const size_t first32 = gsize == 32 ? 0 : groups.size();
+  c->ngroups = (int)groups.size();
+  if (gsize != 32) append_groups(32);
+  c->ngroups32 = (int)(groups.size() - first32);
   dfree(c->groups);
   BH_TRY(dalloc(&c->groups, groups.size()));
-  c->ngroups = (int)groups.size();
+  c->groups32 = c->groups + first32;
   c->batch_group = (int)gsize;
   c->batch_tiles = n <= kBatchTileAny || (n <= kBatchTileMax && largest <= kBatchTileSystem);
   cudaMemcpyAsync(c->sys_off, sys_offsets, sizeof(uint32_t) * (nsys + 1), cudaMemcpyHostToDevice, c->stream);

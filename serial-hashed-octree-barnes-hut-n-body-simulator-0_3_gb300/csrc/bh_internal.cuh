@@ -190,9 +190,12 @@ struct bh_ctx {
   uint32_t* sys_off = nullptr;     // device [nsys + 1]
   uint16_t* body_sys = nullptr;    // device, system of each body slot / tree position
   bh::Geom* sys_geom = nullptr;    // device [nsys]
-  int4* groups = nullptr;          // device walk groups: first body, body count, root node, system
-  int ngroups = 0;
-  int batch_group = 32;            // largest group of the table (32, 16, 8 or 4)
+  // device walk groups (first body, body count, root node, system), of up to batch_group (32, 16, 8 or 4)
+  // bodies; and of up to 32, for the launch shapes of that size (the same table, or the end of the array)
+  int4* groups = nullptr;
+  int4* groups32 = nullptr;
+  int ngroups = 0, ngroups32 = 0;
+  int batch_group = 32;
   bool batch_tiles = false;        // the systems sort in two launches (segments of the tile sort)
   size_t sys_cap = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // captured batched step, by state parity

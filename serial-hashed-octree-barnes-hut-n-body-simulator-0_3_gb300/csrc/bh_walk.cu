@@ -783,13 +783,15 @@ struct WalkArgs {
 
 template <bool kQuad, bool kSelf, class Cfg = CfgDefault, int kGroup = 32>
 void launch_walk_t(bh_ctx* c, int n, const WalkArgs& a) {
-  const int ngroups = a.batch ? c->ngroups : (n + kGroup - 1) / kGroup;
+  const bool own = kGroup == c->batch_group;  // else a shape of groups of 32 on a smaller ensemble
+  const int4* table = !a.batch ? nullptr : own ? c->groups : c->groups32;
+  const int ngroups = !a.batch ? (n + kGroup - 1) / kGroup : own ? c->ngroups : c->ngroups32;
   // every resident block, or a block per group when there are fewer groups than that: the warps
   // that find no group leave, the others spread over all the SMs
   const int grid = min(walk_grid<kQuad, kSelf, false, Cfg, kGroup>(), ngroups);
   k_walk<kQuad, kSelf, false, Cfg, kGroup><<<grid, Cfg::kThreads, 0, c->stream>>>(
       c->wnode, c->tpos, c->tslot, n, a.theta2, a.eps2, a.acc_slot, a.vel_kick, a.half_dt, a.vel_copy,
-      a.batch ? c->groups : nullptr, c->ngroups, c->counters, c->err);
+      table, ngroups, c->counters, c->err);
 }
 
 // The walk with groups of `group` bodies (32, 16, 8 or 4; an ensemble's table is built for it).
@@ -813,10 +815,11 @@ using Cfg4 = WalkCfg<4, 6, 384>;
 using Cfg5 = WalkCfg<4, 8, 512>;
 using Cfg6 = WalkCfg<8, 4, 384, 1>;
 using Cfg7 = WalkCfg<4, 8, 384, 1>;
-// Variant 0, the default, takes its group size from the number of bodies (walk_group_size);
-// variants 8 and 9 fix it to 16 and 8, and 10 and 11 do so at 104 registers (two 8-warp blocks per
-// SM): small single systems, where a few warps per SM walk and the walk's time is one warp's chain
-// of dependent latencies. Ensembles walk their fixed table, whatever the variant's group.
+// Variant 0, the default, takes its group size from the number of bodies (walk_group_size), 1 to 7 walk
+// groups of 32; variants 8 and 9 take 16 and 8, and 10 and 11 do so at 104 registers (two 8-warp blocks
+// per SM): small single systems, where a few warps per SM walk and the walk's time is one warp's chain
+// of dependent latencies. Ensembles have tables of the default's groups and of groups of 32, so for them
+// 8 to 11 are variant 0.
 constexpr int kVariants = 12;
 
 // The 104-register shape of the small groups, while about one wave of its blocks (16 warps per SM)
@@ -845,11 +848,6 @@ void launch_quad_default(bh_ctx* c, int n, const WalkArgs& a, int group) {
 }
 
 void launch_quad_variant(bh_ctx* c, int v, int n, const WalkArgs& a) {
-  const int table = a.batch ? c->batch_group : 0;
-  if (a.batch && table != 32) {  // small ensembles: the table's own group size, default shape
-    launch_quad_default(c, n, a, table);
-    return;
-  }
   if (a.batch && v >= 8) v = 0;
   switch (v) {
     case 1: launch_walk_t<true, false, Cfg1>(c, n, a); break;
@@ -863,7 +861,7 @@ void launch_quad_variant(bh_ctx* c, int v, int n, const WalkArgs& a) {
     case 9: launch_walk_t<true, false, CfgDefault, 8>(c, n, a); break;
     case 10: launch_walk_t<true, false, Cfg2, 16>(c, n, a); break;
     case 11: launch_walk_t<true, false, Cfg2, 8>(c, n, a); break;
-    default: launch_quad_default(c, n, a, a.batch ? 32 : walk_group_size(n)); break;
+    default: launch_quad_default(c, n, a, a.batch ? c->batch_group : walk_group_size(n)); break;
   }
 }
 
