@@ -1313,13 +1313,13 @@ bh_status bh_autotune_walk(bh_ctx* c, double theta, double eps, int trials, bh_t
   float best_ms = 0.f;
   int best = 0;
   for (int v = 0; v < nv; ++v) {
-    const bh::WalkVariant info = bh::walk_variant_info(v, c->n);
+    const bh::WalkVariant info = bh::walk_variant_info(c, v);
     out->warps_per_block[v] = info.warps;
     out->min_blocks_per_sm[v] = info.min_blocks;
     out->stack_depth[v] = info.stack;
     out->cell_form[v] = info.form;
     out->registers[v] = info.regs;
-    out->group_size[v] = batch ? c->batch_group : info.group;  // ensembles walk their fixed group table
+    out->group_size[v] = info.group;
     std::vector<float> ms;
     uint32_t e = 0;
     for (int t = 0; t <= trials && e == 0; ++t) {  // trial 0 warms up

@@ -320,10 +320,11 @@ void launch_fp32_peak(cudaStream_t st, float* sink, int blocks);
 void launch_potential(bh_ctx* c, int n, float theta, float eps, int mode, float* pot_slot);
 // Launch shapes of the quadrupole walk (positive softening) that bh_autotune_walk times.
 struct WalkVariant {
-  int warps, min_blocks, stack, form, regs, group;  // group: bodies per warp (single systems)
+  int warps, min_blocks, stack, form, regs, group;  // group: bodies per warp
 };
 int walk_variants();
-WalkVariant walk_variant_info(int v, size_t n);
+// What variant v launches for the context's present system or ensemble.
+WalkVariant walk_variant_info(const bh_ctx* c, int v);
 // Bodies per walk group for n bodies in all (a single system, or the systems of an ensemble).
 int walk_group_size(size_t n);
 // Bodies per group of the differentiable path's walks.

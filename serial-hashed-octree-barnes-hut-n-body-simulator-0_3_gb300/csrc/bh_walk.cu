@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bh_internal.cuh"
 
@@ -795,13 +796,13 @@ void launch_walk_t(bh_ctx* c, int n, const WalkArgs& a) {
 }
 
 // The walk with groups of `group` bodies (32, 16, 8 or 4; an ensemble's table is built for it).
-template <bool kQuad, bool kSelf, class Cfg = CfgDefault>
+template <bool kQuad, bool kSelf>
 void launch_walk_group(bh_ctx* c, int n, const WalkArgs& a, int group) {
   switch (group) {
-    case 4: launch_walk_t<kQuad, kSelf, Cfg, 4>(c, n, a); break;
-    case 8: launch_walk_t<kQuad, kSelf, Cfg, 8>(c, n, a); break;
-    case 16: launch_walk_t<kQuad, kSelf, Cfg, 16>(c, n, a); break;
-    default: launch_walk_t<kQuad, kSelf, Cfg, 32>(c, n, a); break;
+    case 4: launch_walk_t<kQuad, kSelf, CfgDefault, 4>(c, n, a); break;
+    case 8: launch_walk_t<kQuad, kSelf, CfgDefault, 8>(c, n, a); break;
+    case 16: launch_walk_t<kQuad, kSelf, CfgDefault, 16>(c, n, a); break;
+    default: launch_walk_t<kQuad, kSelf, CfgDefault, 32>(c, n, a); break;
   }
 }
 
@@ -837,14 +838,24 @@ WalkVariant variant_info() {
   return {Cfg::kWarps, Cfg::kMinBlocks, Cfg::kStack, Cfg::kForm, fa.numRegs, kGroup};
 }
 
-// The default shape at a group size: 104 registers while the groups are few (see walk_wide).
+// f(shape, group size) with the default shape for that many groups of `group` bodies: 104 registers while
+// the groups are few (see walk_wide), 80 for groups of 16 (65 536 bodies 409 -> 369 us), else 64.
+template <class F>
+auto with_default_shape(int ngroups, int group, F f) {
+  using std::integral_constant;
+  const bool wide = walk_wide(ngroups, group);
+  switch (group) {
+    case 4: return wide ? f(Cfg2{}, integral_constant<int, 4>{}) : f(CfgDefault{}, integral_constant<int, 4>{});
+    case 8: return wide ? f(Cfg2{}, integral_constant<int, 8>{}) : f(CfgDefault{}, integral_constant<int, 8>{});
+    case 16: return wide ? f(Cfg2{}, integral_constant<int, 16>{}) : f(Cfg1{}, integral_constant<int, 16>{});
+    default: return f(CfgDefault{}, integral_constant<int, 32>{});
+  }
+}
+
 void launch_quad_default(bh_ctx* c, int n, const WalkArgs& a, int group) {
-  if (walk_wide(a.batch ? c->ngroups : (n + group - 1) / group, group))
-    launch_walk_group<true, false, Cfg2>(c, n, a, group);
-  else if (group == 16)
-    launch_walk_t<true, false, Cfg1, 16>(c, n, a);  // 80 registers: 65 536 bodies 409 -> 369 us
-  else
-    launch_walk_group<true, false>(c, n, a, group);
+  with_default_shape(a.batch ? c->ngroups : (n + group - 1) / group, group, [&](auto cfg, auto g) {
+    launch_walk_t<true, false, decltype(cfg), decltype(g)::value>(c, n, a);
+  });
 }
 
 void launch_quad_variant(bh_ctx* c, int v, int n, const WalkArgs& a) {
@@ -912,7 +923,8 @@ int walk_group_size(size_t n) {
   return n < 196608 ? 16 : 32;
 }
 
-WalkVariant walk_variant_info(int v, size_t n) {
+WalkVariant walk_variant_info(const bh_ctx* c, int v) {
+  if (c->batch && v >= 8) v = 0;  // as in launch_quad_variant
   switch (v) {
     case 1: return variant_info<Cfg1>();
     case 2: return variant_info<Cfg2>();
@@ -925,14 +937,12 @@ WalkVariant walk_variant_info(int v, size_t n) {
     case 9: return variant_info<CfgDefault, 8>();
     case 10: return variant_info<Cfg2, 16>();
     case 11: return variant_info<Cfg2, 8>();
-    default:
-      switch (walk_group_size(n)) {
-        case 4: return variant_info<CfgDefault, 4>();
-        case 8: return variant_info<CfgDefault, 8>();
-        case 16: return variant_info<Cfg1, 16>();
-        default: return variant_info<CfgDefault>();
-      }
+    default: break;
   }
+  const int group = c->batch ? c->batch_group : walk_group_size(c->n);
+  const int ngroups = c->batch ? c->ngroups : (int)((c->n + group - 1) / group);
+  return with_default_shape(ngroups, group,
+                            [](auto cfg, auto g) { return variant_info<decltype(cfg), decltype(g)::value>(); });
 }
 
 // One force-only walk with the given variant (the autotuner's trial); acc_out by slot.

@@ -1,4 +1,5 @@
-"""Launch shapes of the walk: a pinned shape is the one that runs, for ensembles and small systems too."""
+"""Launch shapes of the walk for ensembles and small systems: a pinned shape is the one that runs, and the
+autotuner reports the shapes that it timed."""
 import numpy as np
 import pytest
 
@@ -35,3 +36,34 @@ def test_pinned_shape_runs_on_small_ensembles(bh, sizes):
     for a, cells, points in acc[1:]:  # the reference's interaction sets all the same
         assert cells == acc[0][1] and points == acc[0][2]
         assert float(np.median(relerr(a, acc[0][0]))) < 1e-5
+
+
+@pytest.mark.parametrize("sizes,group", list(zip(SIZES, (4, 8, 16))))
+def test_ensemble_rows_are_what_ran(bh, sizes, group):
+    pm, vel, off = ensemble(bh, sizes)
+    prm = bh.default_params(theta=0.6, eps=0.01, dt=1e-3, leaf_capacity=4)
+    with bh.Simulation(len(pm)) as sim:
+        sim.batch_set(pm, vel, off)
+        sim.batch_step(prm, 1)
+        v = sim.autotune(0.6, 0.01, trials=2)["variants"]
+    assert [x["group_size"] for x in v] == [group] + [32] * 7 + [group] * 4
+    shape = [{k: x[k] for k in x if k != "ms"} for x in v]
+    assert all(x == shape[0] for x in shape[8:])
+
+
+@pytest.mark.parametrize("n,shape", [
+    (2000, (2, 4)), (12287, (2, 4)), (12288, (2, 8)), (24575, (2, 8)), (49152, (2, 16)), (49153, (3, 16)),
+    (196607, (3, 16)), (196608, (4, 32)),
+])
+def test_default_row_names_its_kernel(bh, n, shape):
+    """Row 0 against the rows of the pinned shapes with the same registers: 10 and 11 (two blocks per SM),
+    1 (three), 2 (two)."""
+    pm, vel = bh.plummer(2, n)
+    with bh.Simulation(n) as sim:
+        sim.set_bodies(pm, vel)
+        c, size = sim.bounds()
+        sim.build(c, 2 * size, 16, 1)
+        v = sim.autotune(1.0, 0.01, trials=1)["variants"]
+    assert (v[0]["min_blocks_per_sm"], v[0]["group_size"]) == shape
+    # registers a thread within the budget of that many blocks of 256 on the SM's 65 536
+    assert 65536 // 256 // (shape[0] + 1) // 8 * 8 < v[0]["registers"] <= 65536 // 256 // shape[0]
