@@ -275,12 +275,12 @@ bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t* vals_in, 
  * launch shape of the quadrupole tree walk (warps per block, register budget as resident blocks
  * per SM, per-warp stack depth, cell-evaluation form, and bodies per warp group: shape 0, the
  * default, takes 32, 16, 8 or 4 by the number of bodies, shapes 8 to 11 fix 16 or 8, the others 32;
- * a group never exceeds the 32 lanes of a warp, whose opening masks are 32-bit; ensembles walk
- * their fixed table of groups, sized by their number of bodies in all) on the tree currently in
- * the context: the last bh_step / bh_build, or the last bh_batch_step of an ensemble. Each shape runs `trials` timed
- * force-only walks after one warm-up (the state is not changed); the fastest median becomes the
- * context's walk for quadrupole steps with eps > 0. Shapes whose stack cannot hold the tree get
- * ms = -1. */
+ * a group never exceeds the 32 lanes of a warp, whose opening masks are 32-bit; ensembles take
+ * shape 0's groups by their number of bodies in all, and shapes 8 to 11 are shape 0 for them) on the
+ * tree currently in the context: the last bh_step / bh_build, or the last bh_batch_step of an ensemble.
+ * Each shape runs `trials` timed force-only walks after one warm-up (the state is not changed); the
+ * fastest median becomes the context's walk for quadrupole steps with eps > 0, of single systems or of
+ * ensembles, as the tree was. Shapes whose stack cannot hold the tree get ms = -1. */
 #define BH_TUNE_MAX_VARIANTS 12
 typedef struct bh_tune_result {
   int variants;
@@ -294,7 +294,8 @@ typedef struct bh_tune_result {
   float ms[BH_TUNE_MAX_VARIANTS];
 } bh_tune_result;
 bh_status bh_autotune_walk(bh_ctx* ctx, double theta, double eps, int trials, bh_tune_result* out);
-/* Pins the walk's launch shape (an index of bh_tune_result, 0 = the default) without timing. */
+/* Pins the walk's launch shape (an index of bh_tune_result, 0 = the default) without timing, for single
+ * systems and ensembles. */
 bh_status bh_set_walk_variant(bh_ctx* ctx, int variant);
 
 /* Conservation diagnostics of the current state (no counterpart in the reference, which reports

@@ -1320,6 +1320,10 @@ bh_status bh_autotune_walk(bh_ctx* c, double theta, double eps, int trials, bh_t
     out->cell_form[v] = info.form;
     out->registers[v] = info.regs;
     out->group_size[v] = info.group;
+    if (batch && v >= 8) {  // variant 0 again: its time, not another sample of it
+      out->ms[v] = out->ms[0];
+      continue;
+    }
     std::vector<float> ms;
     uint32_t e = 0;
     for (int t = 0; t <= trials && e == 0; ++t) {  // trial 0 warms up
@@ -1349,8 +1353,9 @@ bh_status bh_autotune_walk(bh_ctx* c, double theta, double eps, int trials, bh_t
   if (best_ms == 0.f) return BH_ERR_OVERFLOW_STACK;
   out->variants = nv;
   out->best = best;
-  if (c->walk_variant != best) destroy_graphs(c);  // captured batched steps hold the old kernel
-  c->walk_variant = best;
+  int& kept = batch ? c->batch_variant : c->walk_variant;
+  if (kept != best) destroy_graphs(c);  // captured steps hold the old kernel
+  kept = best;
   clear_device_flags(c);
   return BH_OK;
 }
@@ -1358,8 +1363,8 @@ bh_status bh_autotune_walk(bh_ctx* c, double theta, double eps, int trials, bh_t
 bh_status bh_set_walk_variant(bh_ctx* c, int variant) {
   if (!c || variant < 0 || variant >= std::min(bh::walk_variants(), (int)BH_TUNE_MAX_VARIANTS))
     return BH_ERR_INVALID_ARG;
-  if (c->walk_variant != variant) destroy_graphs(c);
-  c->walk_variant = variant;
+  if (c->walk_variant != variant || c->batch_variant != variant) destroy_graphs(c);
+  c->walk_variant = c->batch_variant = variant;
   return BH_OK;
 }
 

@@ -218,7 +218,8 @@ struct bh_ctx {
 
   void* adj = nullptr;  // differentiable-path state (checkpoints, tape, adjoints): bh_adjoint.cu
 
-  int walk_variant = 0;           // launch shape of the quadrupole walk (bh_autotune_walk)
+  // launch shapes of the quadrupole walk (bh_autotune_walk): single systems, ensembles
+  int walk_variant = 0, batch_variant = 0;
   bool batch_tree_ready = false;  // the arena holds the tree of the last batched step
 };
 

@@ -993,7 +993,7 @@ void launch_walk(bh_ctx* c, int n, float theta, float eps, int mode, float4* acc
   const bool self = !(a.eps2 > 0.f);
   const int group = batch ? c->batch_group : walk_group_size(n);
   if (quad && !self)
-    launch_quad_variant(c, c->walk_variant, n, a);
+    launch_quad_variant(c, batch ? c->batch_variant : c->walk_variant, n, a);
   else if (quad)
     launch_walk_group<true, true>(c, n, a, group);
   else if (self)

@@ -1,5 +1,5 @@
-"""Launch shapes of the walk for ensembles and small systems: a pinned shape is the one that runs, and the
-autotuner reports the shapes that it timed."""
+"""Launch shapes of the walk for ensembles and small systems: a pinned shape is the one that runs, the
+autotuner reports the shapes that it timed, and what it picks for an ensemble stays with ensembles."""
 import numpy as np
 import pytest
 
@@ -45,10 +45,31 @@ def test_ensemble_rows_are_what_ran(bh, sizes, group):
     with bh.Simulation(len(pm)) as sim:
         sim.batch_set(pm, vel, off)
         sim.batch_step(prm, 1)
-        v = sim.autotune(0.6, 0.01, trials=2)["variants"]
+        r = sim.autotune(0.6, 0.01, trials=2)
+    v = r["variants"]
     assert [x["group_size"] for x in v] == [group] + [32] * 7 + [group] * 4
-    shape = [{k: x[k] for k in x if k != "ms"} for x in v]
-    assert all(x == shape[0] for x in shape[8:])
+    assert all(x == v[0] for x in v[8:])  # the same kernel, timed once
+    assert r["best"] < 8 and v[r["best"]]["ms"] == min(x["ms"] for x in v) > 0
+
+
+@pytest.mark.parametrize("pin", [None, 3])
+def test_ensemble_choice_stays_with_ensembles(bh, pin):
+    pm, vel, off = ensemble(bh, SIZES[0])
+    prm = bh.default_params(theta=0.6, eps=0.01, dt=1e-3, leaf_capacity=4)
+    one, onev = bh.plummer(5, 2000)
+    evals = []
+    for tune in (False, True):
+        with bh.Simulation(len(pm)) as sim:
+            if pin is not None:
+                sim.set_walk_variant(pin)
+            if tune:
+                sim.batch_set(pm, vel, off)
+                sim.batch_step(prm, 1)
+                sim.autotune(0.6, 0.01, trials=1)
+            sim.set_bodies(one, onev)
+            st = sim.step(prm, 1)
+            evals.append((st.walk_cell_evals, st.walk_point_evals))
+    assert evals[0] == evals[1]
 
 
 @pytest.mark.parametrize("n,shape", [
