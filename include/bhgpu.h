@@ -255,8 +255,8 @@ bh_status bh_measure_fp32_peak(bh_ctx* ctx, double* tflops);
  * counterpart in the reference. It is meant for callers that cannot call cudaMalloc where
  * they need the sort: per-frame loops and stream-callback chains, where an allocation or free
  * would synchronise the whole device, and embedders with a fixed device-memory budget. The
- * sort's scratch (the tile-sorted keys and values) lives in a fixed device array of the library,
- * which each GPU holds while the library is loaded, so n is limited to
+ * sort's scratch (the partly sorted keys and values, 1.5 MB) lives in a fixed device array of the
+ * library, which each GPU holds while the library is loaded, so n is limited to
  * BH_SORT_STATIC_MAX_KEYS (larger n returns BH_ERR_INVALID_ARG). Sorts stably by the full
  * 64-bit key (the same permutation as bh_sort_bodies) into keys_out / vals_out; the inputs
  * are left unchanged; asynchronous on `stream` (a cudaStream_t, NULL for the legacy default

@@ -324,12 +324,14 @@ auto spans_kernel(const TileShape& sh) {
   return sh.tile == kTileSmall ? k_merge_spans<kTileSmall> : k_merge_spans<kTileSpan>;
 }
 
-// Sorts n pairs by tiles into kout / vout (which may be kin / vin); returns the number of launches.
-int launch_tile_sort(const uint64_t* kin, const uint32_t* vin, uint64_t* ktmp, uint32_t* vtmp, uint64_t* kout,
-                     uint32_t* vout, int n, cudaStream_t st) {
+// Sorts n pairs by tiles into kout / vout (which may be kin / vin); returns the number of launches. With spans
+// there is one more change of buffers, and the tiles go to kfirst / vfirst: the input itself, or memory that
+// overlaps neither it nor ktmp / vtmp.
+int launch_tile_sort(const uint64_t* kin, const uint32_t* vin, uint64_t* kfirst, uint32_t* vfirst, uint64_t* ktmp,
+                     uint32_t* vtmp, uint64_t* kout, uint32_t* vout, int n, cudaStream_t st) {
   const TileShape sh = pairs_shape(n);
-  uint64_t* kt = sh.span ? kout : ktmp;  // with spans one more change of buffers: the tiles start in the output
-  uint32_t* vt = sh.span ? vout : vtmp;
+  uint64_t* kt = sh.span ? kfirst : ktmp;
+  uint32_t* vt = sh.span ? vfirst : vtmp;
   BH_TILE_KERNEL(k_tile_pairs, sh)<<<sh.tile_blocks(), sh.tile, 0, st>>>(kin, vin, kt, vt, n);
   if (sh.span) launch_dependent(spans_kernel(sh), sh.merge_blocks(), kSpanThreads, kt, vt, ktmp, vtmp, n, st);
   launch_dependent(sh.run() == 32 * kTileSmall ? k_merge_pairs<32 * kTileSmall, false> : BH_MERGE_KERNEL(k_merge_pairs, sh),
@@ -369,7 +371,7 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
   if (n <= 1) return;
   if (n <= tile_sort_max() && first_pass == 0 && npasses == kPasses) {
     // the result goes back to keys_in / vals_in, as after the eight digit passes
-    c->launches += launch_tile_sort(keys_in, vals_in, keys_tmp, vals_tmp, keys_in, vals_in, n, st);
+    c->launches += launch_tile_sort(keys_in, vals_in, keys_in, vals_in, keys_tmp, vals_tmp, keys_in, vals_in, n, st);
     return;
   }
   const int tiles = sort_max_tiles((size_t)n);
@@ -408,9 +410,10 @@ void radix_sort_pairs(bh_ctx* c, uint64_t* keys_in, uint32_t* vals_in, uint64_t*
 // a per-frame loop or a chain of stream callbacks, where cudaMalloc / cudaFree would
 // synchronise the whole device and stall other streams, and embedders that reserve a fixed
 // device-memory budget up front and forbid allocations afterwards. For them this variant keeps
-// the scratch the sort needs (the tile-sorted keys and values) in one file-scope __device__ array
-// of fixed size, which the GPU holds for as long as the library is loaded. The caller passes only
-// its inputs and outputs.
+// the scratch the sort needs (the tile-sorted keys and values, and the merged spans') in one
+// file-scope __device__ array of fixed size, which the GPU holds for as long as the library is
+// loaded. The caller passes only its inputs and outputs. The inputs are read in full before an output is
+// written (the first launch writes scratch), so outputs may overlap them in any way.
 //
 // The array's name in host code is only a host-side stand-in for the symbol, not a device
 // address; the device address is resolved with cudaGetSymbolAddress the first time the entry
@@ -425,7 +428,9 @@ namespace {
 constexpr size_t kStaticMaxKeys = BH_SORT_STATIC_MAX_KEYS;
 constexpr size_t kOffTmpKeys = 0;
 constexpr size_t kOffTmpVals = kOffTmpKeys + kStaticMaxKeys * sizeof(uint64_t);
-constexpr size_t kStaticBytes = kOffTmpVals + kStaticMaxKeys * sizeof(uint32_t);
+constexpr size_t kOffFirstKeys = kOffTmpVals + kStaticMaxKeys * sizeof(uint32_t);
+constexpr size_t kOffFirstVals = kOffFirstKeys + kStaticMaxKeys * sizeof(uint64_t);
+constexpr size_t kStaticBytes = kOffFirstVals + kStaticMaxKeys * sizeof(uint32_t);
 
 static __device__ __align__(256) unsigned char g_static_sort_scratch[kStaticBytes];
 
@@ -470,6 +475,7 @@ extern "C" bh_status bh_sort_keys_static(const uint64_t* keys_in, const uint32_t
   }
   uint64_t* tmp_keys = (uint64_t*)(base + kOffTmpKeys);
   uint32_t* tmp_vals = (uint32_t*)(base + kOffTmpVals);
-  launch_tile_sort(keys_in, vals_in, tmp_keys, tmp_vals, keys_out, vals_out, nn, st);
+  launch_tile_sort(keys_in, vals_in, (uint64_t*)(base + kOffFirstKeys), (uint32_t*)(base + kOffFirstVals), tmp_keys,
+                   tmp_vals, keys_out, vals_out, nn, st);
   return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ERR_DEVICE;
 }
