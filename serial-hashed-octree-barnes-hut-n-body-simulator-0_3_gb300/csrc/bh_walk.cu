@@ -776,6 +776,15 @@ int walk_grid() {
   return blocks[dev];
 }
 
+// Blocks of a walk over that many groups, at most. Small groups: a block each, so that they spread over the
+// SMs (a warp's first group goes by its place in the grid; warps that find none leave). Groups of 32, all from
+// the queue: as many warps as groups, since of more the first to arrive would take them, several to an
+// SM (65 536 bodies, shapes 1 / 2 / 3: 460 / 452 / 450 us so, 570 / 452 / 670 with a block each).
+template <class Cfg, int kGroup>
+int walk_blocks(int ngroups) {
+  return kGroup == 32 ? ngroups / Cfg::kWarps + 1 : ngroups;
+}
+
 struct WalkArgs {
   float theta2, eps2, half_dt;
   float4 *acc_slot, *vel_kick, *vel_copy;
@@ -787,9 +796,7 @@ void launch_walk_t(bh_ctx* c, int n, const WalkArgs& a) {
   const bool own = kGroup == c->batch_group;  // else a shape of groups of 32 on a smaller ensemble
   const int4* table = !a.batch ? nullptr : own ? c->groups : c->groups32;
   const int ngroups = !a.batch ? (n + kGroup - 1) / kGroup : own ? c->ngroups : c->ngroups32;
-  // every resident block, or a block per group when there are fewer groups than that: the warps
-  // that find no group leave, the others spread over all the SMs
-  const int grid = min(walk_grid<kQuad, kSelf, false, Cfg, kGroup>(), ngroups);
+  const int grid = min(walk_grid<kQuad, kSelf, false, Cfg, kGroup>(), walk_blocks<Cfg, kGroup>(ngroups));
   k_walk<kQuad, kSelf, false, Cfg, kGroup><<<grid, Cfg::kThreads, 0, c->stream>>>(
       c->wnode, c->tpos, c->tslot, n, a.theta2, a.eps2, a.acc_slot, a.vel_kick, a.half_dt, a.vel_copy,
       table, ngroups, c->counters, c->err);
@@ -885,7 +892,7 @@ namespace {
 template <bool kQuad, int kGroup>
 void launch_potential_t(bh_ctx* c, int n, float theta2, float eps2, float* pot_slot) {
   const int ngroups = (n + kGroup - 1) / kGroup;
-  const int grid = min(walk_grid<kQuad, true, false, CfgDefault, kGroup, true>(), ngroups);
+  const int grid = min(walk_grid<kQuad, true, false, CfgDefault, kGroup, true>(), walk_blocks<CfgDefault, kGroup>(ngroups));
   k_walk<kQuad, true, false, CfgDefault, kGroup, true><<<grid, CfgDefault::kThreads, 0, c->stream>>>(
       c->wnode, c->tpos, c->tslot, n, theta2, eps2, reinterpret_cast<float4*>(pot_slot), nullptr, 0.f, nullptr, nullptr,
       0, c->counters, c->err);
@@ -1009,7 +1016,7 @@ namespace bh {
 template <class Cfg, int kGroup>
 static void launch_walk_record_t(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick,
                                  float half_dt, Chunk* tape, unsigned* tape_count, int tape_cap) {
-  const int grid = min(walk_grid<true, false, true, Cfg, kGroup>(), (n + kGroup - 1) / kGroup);
+  const int grid = min(walk_grid<true, false, true, Cfg, kGroup>(), walk_blocks<Cfg, kGroup>((n + kGroup - 1) / kGroup));
   k_walk<true, false, true, Cfg, kGroup><<<grid, Cfg::kThreads, 0, c->stream>>>(
       c->wnode, c->tpos, c->tslot, n, theta * theta, eps * eps, acc_slot, vel_kick, half_dt, nullptr, nullptr, 0,
       c->counters, c->err, tape, tape_count, tape_cap);

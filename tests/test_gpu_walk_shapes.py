@@ -88,3 +88,15 @@ def test_default_row_names_its_kernel(bh, n, shape):
     assert (v[0]["min_blocks_per_sm"], v[0]["group_size"]) == shape
     # registers a thread within the budget of that many blocks of 256 on the SM's 65 536
     assert 65536 // 256 // (shape[0] + 1) // 8 * 8 < v[0]["registers"] <= 65536 // 256 // shape[0]
+
+
+def test_shapes_of_one_group_size_take_alike(bh):
+    """Groups of 32 on a system with fewer of them than the GPU has warps: every shape spreads them over the
+    SMs. The shapes differ in registers, block size and stack; their walks differ by 3%."""
+    n = 65536
+    pm, vel = bh.plummer(0, n)
+    with bh.Simulation(n) as sim:
+        sim.set_bodies(pm, vel)
+        sim.step(bh.default_params(theta=0.5, eps=0.01, dt=1e-3, leaf_capacity=8), 2)
+        ms = [v["ms"] for v in sim.autotune(0.5, 0.01, trials=15)["variants"][1:8]]
+    assert max(ms) < 1.2 * min(ms)
