@@ -955,9 +955,10 @@ bh_status bh_measure_fp32_peak(bh_ctx* c, double* tflops) {
 // ---------------------------------------------------------------------------------------
 // Batched ensembles: many independent systems in one context, stepped together. Each system
 // keeps a fixed body range [off[s], off[s+1]); every stage runs over all bodies at once:
-// per-system bounds; Morton keys with the system's own cube; a stable sort by key followed by
-// a stable sort by system id, which regroups every system in key order inside its range; the
-// same for tree keys; one tree level build for all systems together (one root per system);
+// per-system bounds; Morton keys with the system's own cube; a stable sort by (system, key), by
+// tiles for small ensembles, else by key and then by system id, which regroups every system in
+// key order inside its range; the same for tree keys; one build of every depth for all systems
+// together (one root per system), or of one level at a time above a leaf capacity of 64;
 // one walk over groups of up to 32 bodies that never straddle a system, pulled from a global
 // work queue. Each step is captured once per state parity in a CUDA graph and replayed.
 // ---------------------------------------------------------------------------------------

@@ -503,7 +503,7 @@ __global__ __launch_bounds__(kTile) void k_tree_tiles(const uint64_t* __restrict
 
 // The half-kick and drift of bodies that keep their slots (the differentiable path), with the tree keys
 // of the drifted positions tile-sorted. The bodies are taken in the previous tree order, in which
-// the new keys are nearly sorted and the merge has little to search (65 536 bodies: 75 -> 35 us
+// the new keys are nearly sorted and the merge has little to search (65 536 bodies: 75 -> 34 us
 // against slot order); bodies of one key keep that order.
 template <int kTile, bool kSeg>
 __global__ __launch_bounds__(kTile) void k_kd_tiles(const float4* __restrict__ pin,

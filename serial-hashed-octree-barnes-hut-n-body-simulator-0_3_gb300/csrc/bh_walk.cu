@@ -831,10 +831,10 @@ using Cfg7 = WalkCfg<4, 8, 384, 1>;
 constexpr int kVariants = 12;
 
 // The 104-register shape of the small groups, while about one wave of its blocks (16 warps per SM)
-// holds them all: a warp then walks one group, and its latency is the walk's. Quadrupole walk, us at
-// 64 / 104 registers: 1 000 bodies in groups of 4 54.3 / 51.6; 10 000 (2 500 groups) 123.7 / 117.9;
-// 16 384 in groups of 8 171.5 / 160.7, of 4 (4 096 groups) 182.8 / 197.0; 65 536 in groups of 16
-// (4 096 groups) 402 / 406.
+// holds them all: a warp then walks one group, and its latency is the walk's. Quadrupole walk, us at 64
+// (groups of 16: 80) / 104 registers: 1 000 bodies in groups of 4 46.7 / 42.7; 10 000 (2 500 groups) 114.5 /
+// 104.0; 16 384 in groups of 8 160.0 / 145.4, of 4 (4 096 groups) 171.8 / 178.7; 32 768 in groups of 16
+// (2 048 groups) 223 / 237, 65 536 (4 096 groups) 360 / 403: for groups of 16 the line could lie lower.
 constexpr int kWideMaxGroups = 3072;
 bool walk_wide(int ngroups, int group) { return group < 32 && ngroups <= kWideMaxGroups; }
 
@@ -846,7 +846,7 @@ WalkVariant variant_info() {
 }
 
 // f(shape, group size) with the default shape for that many groups of `group` bodies: 104 registers while
-// the groups are few (see walk_wide), 80 for groups of 16 (65 536 bodies 409 -> 369 us), else 64.
+// the groups are few (see walk_wide), 80 for groups of 16 (65 536 bodies 417 us at 64, 360 at 80), else 64.
 template <class F>
 auto with_default_shape(int ngroups, int group, F f) {
   using std::integral_constant;
@@ -920,10 +920,10 @@ void launch_potential(bh_ctx* c, int n, float theta, float eps, int mode, float*
 
 // Small groups give more warps and, with their boxes, fewer entries a body (at 16 384 bodies, leaf
 // capacity 1, a group of 32 / 16 / 8 evaluates 2200 / 1835 / 1569 entries), but each group traverses
-// the tree. Quadrupole walk, us with groups of 4 / 8 / 16 / 32 (theta 0.5): 1 000 bodies 52 / 58 / 68 /
-// 134; 10 000 118 / 126 / 159 / 304; 16 384 183 / 161 / 179 / 345; 32 768 298 / 259 / 240 / 351;
-// 65 536 576 / 419 / 402 / 452; 131 072 1104 / 769 / 642 / 741; 262 144 2269 / 1507 / 1210 / 1206.
-// The literal walk crosses at the same sizes.
+// the tree. Quadrupole walk, us with groups of 4 / 8 / 16 / 32, each in its default shape (theta 0.5; leaf
+// capacity 1 up to 16 384 bodies, 8 above): 1 000 bodies 43 / 51 / 66 / 142; 10 000 104 / 116 / 152 / 309;
+// 16 384 172 / 145 / 166 / 352; 32 768 274 / 240 / 237 / 357; 65 536 525 / 401 / 360 / 455; 131 072 1036 /
+// 754 / 668 / 755; 262 144 2125 / 1474 / 1237 / 1200. The literal walk crosses at the same sizes.
 int walk_group_size(size_t n) {
   if (n < 12288) return 4;
   if (n < 24576) return 8;
@@ -1027,7 +1027,8 @@ int record_group_size(size_t n) { return std::min(32, std::max(16, walk_group_si
 
 // The recording walk without its tape, for the forward pass: the same groups whatever the context's variant,
 // so that a recomputed step repeats the forward step's sums bit for bit. (Forward steps in groups of 4 or
-// 8 would walk 10 to 26% faster below 24 576 bodies, but recomputed trajectories would drift away from them.)
+// 8 would walk faster below 24 576 bodies, 1 000 in 43 us instead of 66, 16 384 in 145 instead of 166, but
+// recomputed trajectories would drift away from them.)
 void launch_walk_unrecorded(bh_ctx* c, int n, float theta, float eps, float4* acc_slot, float4* vel_kick,
                             float half_dt) {
   if (n <= 0) return;
