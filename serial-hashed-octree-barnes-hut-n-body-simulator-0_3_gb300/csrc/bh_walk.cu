@@ -239,6 +239,19 @@ __device__ __forceinline__ void eval_points(Smem& s, int cnt, const WalkNode* __
   acc.add(bx, by, bz);
 }
 
+// Arithmetic that keeps denormals, in a file compiled to flush them: a squared distance below 1.2e-38
+// (distances below 1.1e-19) still has an inverse root.
+__device__ __forceinline__ float fma_keep(float a, float b, float c) {
+  float r;
+  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_keep(float x) {
+  float r;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // The potential's terms (diagnostics): M / D + d.Q.d / (2 D^5) of a cell, m / D of a point at another
 // position than the body's. phi = -sum, summed with every rounding error kept and rounded once at
 // the end, so that it does not depend on the order in which a group meets its cells and bodies. The terms
@@ -282,8 +295,9 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
     const int j = r + slot;
     const float4 c0 = s.st0[j], c2 = s.st2[j];
     const float dx = c0.x - px, dy = c0.y - py, dz = c0.z - pz;
-    const float d2 = fmaf(dx, dx, fmaf(dy, dy, kCells ? dz * dz : fmaf(dz, dz, c2.x)));
-    const float rinv = rsqrtf(d2 + (kCells ? eps2 : c2.y));
+    // nodes are accepted at normal squared distances only; bodies may be closer
+    const float rinv = kCells ? rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) + eps2)
+                              : rsqrt_keep(fma_keep(1.f, fma_keep(dx, dx, fma_keep(dy, dy, fma_keep(dz, dz, c2.x))), c2.y));
     bool take = (__float_as_uint(c2.w) & lanebit) != 0u;
     float term;
     if (kCells) {

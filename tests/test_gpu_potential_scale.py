@@ -1,0 +1,30 @@
+"""Potentials of systems whose squared distances are denormal floats (the diagnostics keep them, without a
+softening too), against FP64 direct sums."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("multipole", [0, 1])
+@pytest.mark.parametrize("scale", [1.0, 1e-19, 1e-20])
+def test_potential_at_small_scales(bh, scale, multipole):
+    # a jittered lattice: distances from 0.5 to 11 of the scale, squares down to 2.5e-41, 2e4 denormal steps;
+    # theta 0 takes every pair directly
+    k = 7
+    rng = np.random.default_rng(k)
+    x = np.stack(np.meshgrid(*[np.arange(k) - (k - 1) / 2] * 3, indexing="ij"), -1).reshape(-1, 3)
+    n = len(x)
+    pm = np.zeros((n, 4), np.float32)
+    pm[:, :3] = (x + rng.uniform(-0.2, 0.2, x.shape)) * scale
+    pm[:, 3] = rng.uniform(0.5, 1.5, n) / n
+    with bh.Simulation(n) as sim:
+        sim.set_bodies(pm, np.zeros_like(pm))
+        sim.build(np.zeros(3), 16.0 * scale, 4, multipole)
+        e, pot = sim.energy(0.0, 0.0, potential=True)
+    p = pm.astype(np.float64)
+    r = np.linalg.norm(p[:, None, :3] - p[None, :, :3], axis=-1)
+    np.fill_diagonal(r, np.inf)
+    want = -(p[None, :, 3] / r).sum(1)
+    assert np.abs(pot / want - 1).max() < 1e-4  # half a step of the closest squares: 2.5e-5, half that in 1 / D
+    assert abs(e["potential"] / (0.5 * (p[:, 3] * want).sum()) - 1) < 1e-4
