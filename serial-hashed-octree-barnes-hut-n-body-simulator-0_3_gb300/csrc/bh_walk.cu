@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 #include "bh_internal.cuh"
@@ -96,6 +97,14 @@ struct Acc {
     const float t = sx + x, b = t - sx;
     cx -= (sx - (t - b)) + (x - b);
     sx = t;
+  }
+  // The compensation folded into the sum, the rest of it kept. An infinite sum has no rest (its two-sum
+  // errors are no numbers) and stays infinite.
+  __device__ __forceinline__ void settle() {
+    const float t = sx - cx;
+    const bool infinite = fabsf(sx) > FLT_MAX;
+    cx = infinite ? 0.f : (t - sx) + cx;
+    sx = infinite ? sx : t;
   }
 };
 
@@ -314,9 +323,7 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
     }
     acc.add_exactly(take ? -term : 0.f);
   }
-  const float t = acc.sx - acc.cx;  // the errors stay below half an ulp of the sum
-  acc.cx = (t - acc.sx) + acc.cx;
-  acc.sx = t;
+  acc.settle();  // the errors stay below half an ulp of the sum
 }
 
 // Moves buffer entries [32, n) to [0, n - 32) after the first 32 were evaluated.
@@ -717,7 +724,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         acc.cx += oc;
         acc.add_exactly(os);
       }
-      acc.sx -= acc.cx;
+      acc.settle();
     } else if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
 #pragma unroll
       for (int o = kGroup; o < 32; o <<= 1) {

@@ -28,3 +28,21 @@ def test_potential_at_small_scales(bh, scale, multipole):
     want = -(p[None, :, 3] / r).sum(1)
     assert np.abs(pot / want - 1).max() < 1e-4  # half a step of the closest squares: 2.5e-5, half that in 1 / D
     assert abs(e["potential"] / (0.5 * (p[:, 3] * want).sum()) - 1) < 1e-4
+
+
+@pytest.mark.parametrize("others", [0, 5, 13000])
+def test_overflowing_pair(bh, others):
+    """Two bodies whose m / D is no float have infinite potentials, not ones that are no numbers; a far body's
+    stay finite."""
+    n = 2 + others
+    rng = np.random.default_rng(others)
+    pm = np.zeros((n, 4), np.float32)
+    pm[:, :3] = rng.uniform(-1, 1, (n, 3))
+    pm[:, 3] = 1.0
+    pm[0], pm[1] = (1e-10, 0, 0, 1e30), (-1e-10, 0, 0, 1e30)
+    with bh.Simulation(n) as sim:
+        sim.set_bodies(pm, np.zeros_like(pm))
+        sim.build(np.zeros(3), 2.5, 4, 1)
+        e, pot = sim.energy(0.0, 0.0, potential=True)
+    assert np.array_equal(pot[:2], [-np.inf, -np.inf]) and np.isfinite(pot[2:]).all()
+    assert e["potential"] == -np.inf
