@@ -326,6 +326,14 @@ __device__ __forceinline__ void eval_potential(Smem& s, int cnt, const WalkNode*
   acc.settle();  // the errors stay below half an ulp of the sum
 }
 
+// The plain sum of a body's slots, in all of them.
+template <int kGroup>
+__device__ __forceinline__ float slot_sum(float x) {
+#pragma unroll
+  for (int o = kGroup; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
 // Moves buffer entries [32, n) to [0, n - 32) after the first 32 were evaluated.
 __device__ __forceinline__ void shift_down(int* idx, uint32_t* msk, int n, int lane) {
   __syncwarp();
@@ -726,6 +734,7 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
       }
       acc.settle();
     } else if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
+      const float sx = acc.sx, sy = acc.sy, sz = acc.sz;
 #pragma unroll
       for (int o = kGroup; o < 32; o <<= 1) {
         const float ox = __shfl_xor_sync(0xffffffffu, acc.sx, o), oy = __shfl_xor_sync(0xffffffffu, acc.sy, o),
@@ -736,6 +745,13 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         acc.cy += ey;
         acc.cz += ez;
         acc.add(ox, oy, oz);
+      }
+      // an infinite slot's compensation is no number: the sum of the slots without it, for that body
+      if (__any_sync(0xffffffffu, !(fabsf(acc.sx) + fabsf(acc.sy) + fabsf(acc.sz) <= FLT_MAX))) {
+        const float tx = slot_sum<kGroup>(sx), ty = slot_sum<kGroup>(sy), tz = slot_sum<kGroup>(sz);
+        if (acc.sx != acc.sx) acc.sx = tx;
+        if (acc.sy != acc.sy) acc.sy = ty;
+        if (acc.sz != acc.sz) acc.sz = tz;
       }
     }
     if (kPot) {  // acc_slot receives one float per body
