@@ -1,5 +1,6 @@
-"""Potentials of systems whose squared distances are denormal floats (the diagnostics keep them, without a
-softening too), against FP64 direct sums."""
+"""Potentials at scales where factors of their terms are denormal floats, which the diagnostics keep: squared
+distances of tiny systems, without a softening too, against FP64 direct sums; and 1 / D^5 of the cells' quadrupoles in
+large ones, against the same system at another scale."""
 import numpy as np
 import pytest
 
@@ -28,6 +29,24 @@ def test_potential_at_small_scales(bh, scale, multipole):
     want = -(p[None, :, 3] / r).sum(1)
     assert np.abs(pot / want - 1).max() < 1e-4  # half a step of the closest squares: 2.5e-5, half that in 1 / D
     assert abs(e["potential"] / (0.5 * (p[:, 3] * want).sum()) - 1) < 1e-4
+
+
+def test_quadrupoles_at_large_scales(bh):
+    # 2^25: a change of exponents only, so the potentials are the same times 2^-25 but for 1 / D^5, which is
+    # denormal for D above 1.2 of the scale. Below 8 of it its half step is 2^-10 of it, and the quadrupole terms are
+    # a few hundredths of a potential at theta 1.
+    n, scale = 1000, 2.0**25
+    pm, vel = bh.plummer(6, n)
+    pot = []
+    for k in (1.0, scale):
+        p = pm.copy()
+        p[:, :3] *= np.float32(k)
+        with bh.Simulation(n) as sim:
+            sim.set_bodies(p, vel)
+            c, size = sim.bounds()
+            sim.build(c, 2 * size, 4, 1)
+            pot.append(sim.energy(1.0, 0.0, potential=True)[1] * k)
+    assert np.linalg.norm(pot[1] - pot[0]) < 1e-4 * np.linalg.norm(pot[0])
 
 
 @pytest.mark.parametrize("others", [0, 5, 13000])
