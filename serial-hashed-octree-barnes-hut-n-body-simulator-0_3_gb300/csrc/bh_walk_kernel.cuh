@@ -91,6 +91,21 @@ struct Acc {
     cz = (t - sz) - y;
     sz = t;
   }
+  // The sums of all the slots of a body, in each of them.
+  template <int kGroup>
+  __device__ __forceinline__ void add_slots() {
+#pragma unroll
+    for (int o = kGroup; o < 32; o <<= 1) {
+      const float ox = __shfl_xor_sync(0xffffffffu, sx, o), oy = __shfl_xor_sync(0xffffffffu, sy, o),
+                  oz = __shfl_xor_sync(0xffffffffu, sz, o);
+      const float ex = __shfl_xor_sync(0xffffffffu, cx, o), ey = __shfl_xor_sync(0xffffffffu, cy, o),
+                  ez = __shfl_xor_sync(0xffffffffu, cz, o);
+      cx += ex;
+      cy += ey;
+      cz += ez;
+      add(ox, oy, oz);
+    }
+  }
   // x to the first sum, its rounding error to the first compensation (two-sum, whichever is larger)
   __device__ __forceinline__ void add_exactly(float x) {
     const float t = sx + x, b = t - sx;
@@ -718,22 +733,14 @@ __global__ __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) void k_walk(const W
         acc.add_exactly(os);
       }
       acc.settle();
-    } else if (kSlots > 1) {  // the slots' sums of each body, compensated like the flushes
-      const float sx = acc.sx, sy = acc.sy, sz = acc.sz;
-#pragma unroll
-      for (int o = kGroup; o < 32; o <<= 1) {
-        const float ox = __shfl_xor_sync(0xffffffffu, acc.sx, o), oy = __shfl_xor_sync(0xffffffffu, acc.sy, o),
-                    oz = __shfl_xor_sync(0xffffffffu, acc.sz, o);
-        const float ex = __shfl_xor_sync(0xffffffffu, acc.cx, o), ey = __shfl_xor_sync(0xffffffffu, acc.cy, o),
-                    ez = __shfl_xor_sync(0xffffffffu, acc.cz, o);
-        acc.cx += ex;
-        acc.cy += ey;
-        acc.cz += ez;
-        acc.add(ox, oy, oz);
-      }
-      // an infinite slot's compensation is no number: the sum of the slots without it, for that body
-      if (__any_sync(0xffffffffu, !(fabsf(acc.sx) + fabsf(acc.sy) + fabsf(acc.sz) <= FLT_MAX))) {
-        const float tx = slot_sum<kGroup>(sx), ty = slot_sum<kGroup>(sy), tz = slot_sum<kGroup>(sz);
+    } else if (kSlots > 1) {
+      // the slots' sums of each body, compensated like the flushes; an infinite slot's compensation is no
+      // number, so a body that has one takes the plain sum
+      if (__all_sync(0xffffffffu, fabsf(acc.sx) + fabsf(acc.sy) + fabsf(acc.sz) <= FLT_MAX)) {
+        acc.add_slots<kGroup>();
+      } else {
+        const float tx = slot_sum<kGroup>(acc.sx), ty = slot_sum<kGroup>(acc.sy), tz = slot_sum<kGroup>(acc.sz);
+        acc.add_slots<kGroup>();
         if (acc.sx != acc.sx) acc.sx = tx;
         if (acc.sy != acc.sy) acc.sy = ty;
         if (acc.sz != acc.sz) acc.sz = tz;
